@@ -44,12 +44,9 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
 BYTES_PER_CROSSING = 32  # FP64 n, x read + J read-modify-write per crossing
-# DRAM bytes (read + write) per walk launch, averaged over the 12 walk launches
-# of one iteration of the default workload (1e7 packets), from an ncu capture
-# of `bench.py --steps 3 --warmup 3` (k_walk32: FP32 walk, k_walkm: mixed walk);
-# other workloads and settings were not captured and report null.
-WALK_TRAFFIC_PER_LAUNCH = {("lognormal128", 1e7, "fp32"): 94.02e6,
-                           ("lognormal128", 1e7, "mixed"): 207.79e6}
+# DRAM bytes (read + write) per walk launch of the default workload, from an ncu
+# capture; workloads and settings that were not captured report null.
+WALK_TRAFFIC_PER_LAUNCH = {}
 METRIC = "cell-crossings/s"  # plus time to converged x_H, warm start vs plain ("warm_start")
 UNIT = "crossings/s"
 DESCRIPTIONS = {
@@ -534,8 +531,7 @@ def ours(args):
     peak, peak_kind = measured_peak_hbm()
     total_kt = sum(v[0] for v in kt.values())
     roofline = {
-        "kernel": {"fp32": "k_walk32", "mixed": "k_walkm",
-                   "fp64": "k_walk64"}[args.precision] + " (transport round)",
+        "kernel": "k_path (emission and walk, %s)" % args.precision,
         "bound": "hbm", "achieved": achieved,
         "peak": peak, "unit": "GB/s", "frac": achieved / peak, "peak_source": peak_kind,
         "traffic": WALK_TRAFFIC_PER_LAUNCH.get((args.workload, wl.total_packets, args.precision)),

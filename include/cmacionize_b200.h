@@ -117,6 +117,9 @@ typedef struct {
   int32_t rng;                 /* cmi_rng */
   int32_t device;              /* CUDA device ordinal */
   int32_t threads_per_cta;     /* 0 = library default (256) */
+  /* the next and packets_per_chunk, max_run_chunks, refill_lanes shape the wavefront, which
+   * carries cmi_transport_packets and, with CMI_RNG_RANLUX or FP32 tallies, the iterations;
+   * the other iterations follow each packet's whole path in one kernel */
   int32_t ctas_per_sm;         /* 0 = as many as fit */
   int32_t packets_per_chunk;   /* 0 = library default (128; 256 when subgrids have <= 1024
                                   cells); power of two in [32, 4096] */
@@ -138,7 +141,7 @@ typedef struct {
   uint64_t subgrid_transits; /* calls of interact */
   double mean_abs_dx;        /* mean |x_new - x_old| over the cells of the instance */
   uint32_t error_flags;      /* CMI_FLAG_* bits raised on the device */
-  uint32_t rounds;           /* wavefront rounds that carried packets */
+  uint32_t rounds;           /* most subgrids a packet of the context visited (wavefront rounds) */
   uint64_t packets_reemitted; /* absorptions followed by a reemission */
 } cmi_stats;
 
@@ -169,9 +172,8 @@ int cmi_set_fields(cmi_context *context, int32_t instance, int32_t layout, int32
  * the previous iteration's x_H comes back (cmi_get_fields), and
  * cmi_set_fields_prefetched then takes it together with x_H (host or device,
  * `memory`) in the prefetch's layout.  cmi_set_fields_prefetched returns
- * without waiting: its copies run on the side stream while the next
- * iteration emits its packets, and the iteration's first transport round
- * waits for them.  Both input arrays must stay unchanged until the next
+ * without waiting: its copies run on the side stream, and the next
+ * iteration's transport waits for them.  Both input arrays must stay unchanged until the next
  * cmi_run_iterations, cmi_run_until_converged, cmi_shoot_packets,
  * cmi_get_fields or cmi_synchronize returns; every other entry point orders
  * its own work after the copies.  One prefetch per instance may be pending.
@@ -299,7 +301,8 @@ int cmi_last_launch_count(cmi_context *context, uint64_t *launches);
  * iterations are launched kernel by kernel (no graph) with an event pair
  * around every launch; cmi_kernel_timing returns the summed device time (ms)
  * and launch count of each kernel class since the last call:
- * [0] walk, [1] plan + scatter, [2] emission, [3] balance. */
+ * [0] walk (whole paths: emission included), [1] plan + scatter and [2] emission
+ * (wavefront only), [3] balance. */
 #define CMI_KERNEL_CLASSES 4
 int cmi_set_kernel_timing(cmi_context *context, int32_t enable);
 int cmi_kernel_timing(cmi_context *context, double milliseconds[CMI_KERNEL_CLASSES],

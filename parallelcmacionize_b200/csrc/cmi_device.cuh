@@ -93,6 +93,7 @@ struct alignas(16) DevInstance {
   int64_t num_cells;
   uint32_t frozen;        // 1: converged, emits nothing and keeps x_H (run until converged)
   float reemission;       // probability that an absorbed packet is re-emitted
+  double tally_weight;    // J of one fixed-point tally unit, sigma lref / 2^22 (m^3)
 };
 
 struct alignas(16) DevSource {
@@ -121,7 +122,11 @@ struct alignas(16) DevStats {
   unsigned long long reemitted;
 };
 
-// Control block of the wavefront.
+// The packets of an iteration are cut into this many shares; the CTAs of the path
+// kernel start on different ones.
+constexpr int kPathShares = 16;
+
+// Control block of the transport.
 struct alignas(16) RoundState {
   uint32_t chunk_next;     // chunks claimed in this round
   uint32_t num_chunks;     // chunks of this round
@@ -135,6 +140,7 @@ struct alignas(16) RoundState {
   uint32_t capacity;       // arena capacity (packets)
   uint32_t round_index;    // walks started this iteration (graph loop)
   uint32_t pad[2];
+  uint32_t share_next[kPathShares];  // packets claimed of each share (path kernel)
 };
 
 // FP64 packet: the reference Photon layout (80 B); `meta` (the reserved

@@ -5,6 +5,7 @@
 
 #include "cmi_kernels.cuh"
 #include "cmi_dust.cuh"
+#include "cmi_path.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -61,6 +62,13 @@ constexpr int kReemissionRoundCap = 4096;
 // 24 -> 5.69e10)
 constexpr uint32_t kDefaultRefill = 16;
 constexpr uint32_t kDefaultRefillMixed = 12;
+
+// Tally copies of the subgrids near a source (cmi_path.cuh).  B200, log-normal 128^3
+// (4 sources one after another), us per iteration: within 2 cells of a source 8 / 16 /
+// 32 copies 2930 / 2620 / 2360, within 6 cells 2860 / 2285 / 2230; one copy 12000.
+constexpr double kHotCells = 5.;
+constexpr uint32_t kTallyCopies = 16;  // a multiple of 8
+constexpr size_t kHotBytes = 64u << 20;
 
 struct HostInstance {
   cmi_grid_desc desc;
@@ -133,6 +141,17 @@ struct cmi_context {
   double *d_stage = nullptr;
   size_t stage_bytes = 0;
 
+  // whole-path transport (cmi_path.cuh) instead of the wavefront, and what it needs
+  bool path = false;
+  DevGeo *d_geo = nullptr;
+  unsigned long long *d_tally = nullptr;
+  uint32_t *d_hot = nullptr;   // per subgrid: first cell of its tally copies, 0: none
+  uint32_t copies = 1;
+  size_t tally_words = 0, tally_need = 0;
+  int32_t path_table = 0;
+  size_t path_smem = 0;
+  int path_grid[2] = {0, 0};  // CTAs without and with reemission
+
   // walk launch configuration
   int walk_grid = 0;
   size_t walk_smem = 0;
@@ -181,6 +200,7 @@ struct cmi_context {
   size_t dust_pixels = 0;
 
   bool fp32() const { return opt.transport_precision == CMI_TRANSPORT_FP32; }
+  bool fp64() const { return opt.transport_precision == CMI_TRANSPORT_FP64; }
   bool mixed() const { return opt.transport_precision == CMI_TRANSPORT_MIXED; }
   // the FP32 and mixed walks read the FP32 opacity field kappa = sigma n x
   bool uses_kappa() const { return fp32() || mixed(); }
@@ -243,12 +263,17 @@ int timed_launch(cmi_context *c, int cls, F &&launch) {
   return rc;
 }
 
-// Arena for `packets` packets in flight.
+int check_packets(uint64_t packets) {
+  if (packets > 0xF0000000ull)
+    return fail(CMI_ERR_CAPACITY, "%llu packets exceed the 32-bit packet index",
+                (unsigned long long)packets);
+  return CMI_OK;
+}
+
+// Arena for `packets` packets in flight (wavefront).
 int ensure_capacity(cmi_context *c, uint64_t packets) {
   if (packets <= c->capacity && c->d_arena_in) return CMI_OK;
-  if (packets > 0xF0000000ull)
-    return fail(CMI_ERR_CAPACITY, "%llu packets exceed the 32-bit arena index",
-                (unsigned long long)packets);
+  CMI_TRY(check_packets(packets));
   const uint64_t cap = std::max<uint64_t>(packets, 1024);
   free_graph(c);
   dev_free(c->d_arena_in);
@@ -285,6 +310,116 @@ uint64_t total_budget(const cmi_context *c) {
   return n;
 }
 
+DevGeo instance_geometry(const cmi_context *c, const HostInstance &I) {
+  const DevSubgrid &S = c->h_sub[I.first_sub];
+  DevGeo g{};
+  float lref = 0.f;
+  int32_t off = 0;
+  for (int a = 0; a < 3; ++a) {
+    g.cs[a] = S.cell_size[a];
+    g.inv_cs[a] = S.inv_cell_size[a];
+    g.cs_f[a] = S.cell_size_f[a];
+    g.inv_cs_f[a] = (float)S.inv_cell_size[a];
+    g.n[a] = S.ncell[a];
+    g.ns[a] = I.desc.num_subgrid[a];
+    lref = std::max(lref, S.cell_size_f[a]);
+    g.face_off[a] = off;
+    off += g.n[a] + 3;
+  }
+  for (int a = 0; a < 3; ++a) {
+    g.anchor_off[a] = off;
+    off += g.ns[a] + 2;
+  }
+  g.inf_off = off++;
+  g.table = off;
+  g.sigma = I.desc.cross_section;
+  g.reemission = (double)(float)I.reemission;
+  g.padded = (uint32_t)I.padded_per_sub;
+  for (int a = 0; a < 3; ++a) {
+    g.stride[a] = a == 0 ? g.n[1] * g.n[2] : (a == 1 ? g.n[2] : 1);
+    g.sub_stride[a] = a == 0 ? g.ns[1] * g.ns[2] : (a == 1 ? g.ns[2] : 1);
+    g.jump[a] = g.sub_stride[a] * I.padded_per_sub - g.n[a] * g.stride[a];
+  }
+  g.first_cell = (uint32_t)I.first_cell;
+  g.first_sub = I.first_sub;
+  g.tally_scale = 4194304.f / lref;
+  return g;
+}
+
+// Subgrids with copies of their tally (cmi_path.cuh): those within `radius` cells of
+// a source, with as many copies as pay; fewer cells rather than fewer than eight
+// copies, none if even eight copies of the sources' own subgrids cost more than they
+// save.  hot[s]: first word of the copies of subgrid s.
+//   cost: the balance reads every copy, at about 2e12 bytes a second;
+//   saving: the line through a source takes about 1.5 reductions of each of its
+//   packets, 1.7e9 a second (measured: 16 hot cells in one line).
+int plan_tally_copies(cmi_context *c, std::vector<uint32_t> &hot) {
+  std::vector<uint32_t> list;
+  uint32_t copies = 1;
+  double most = 0.;  // packets of the source with the most
+  for (const HostInstance &I : c->inst) {
+    double total = 0.;
+    for (double l : I.src_lum) total += l;
+    for (double l : I.src_lum) most = std::max(most, l / total * (double)I.num_photon);
+  }
+  const double pays = std::min(1.5 * most / 1.7e9 * 2e12, (double)kHotBytes);  // bytes
+  for (double radius : {kHotCells, 2., 0.}) {
+    hot.assign(c->S, 0u);
+    list.clear();
+    size_t cells = 0;
+    for (const HostInstance &I : c->inst) {
+      const int32_t *ns = I.desc.num_subgrid;
+      for (size_t k = 0; k < I.src_lum.size(); ++k) {
+        int lo[3], hi[3];
+        for (int a = 0; a < 3; ++a) {
+          const double u = (I.src_pos[3 * k + a] - I.desc.box[a]) / I.desc.box[3 + a] *
+                           I.desc.ncell[a];  // in cells
+          const int m = I.sub_ncell[a];
+          lo[a] = std::min(ns[a] - 1, std::max(0, (int)std::floor((u - radius) / m)));
+          hi[a] = std::min(ns[a] - 1, std::max(0, (int)std::floor((u + radius) / m)));
+        }
+        for (int x = lo[0]; x <= hi[0]; ++x)
+          for (int y = lo[1]; y <= hi[1]; ++y)
+            for (int z = lo[2]; z <= hi[2]; ++z) {
+              const uint32_t sub = I.first_sub + (uint32_t)((x * ns[1] + y) * ns[2] + z);
+              if (hot[sub]) continue;
+              hot[sub] = 1u;
+              list.push_back(sub);
+              cells += (size_t)I.padded_per_sub;
+            }
+      }
+    }
+    copies = kTallyCopies;
+    while (copies >= 8 && ((double)(cells * copies * 8) > pays ||
+                           c->total_padded + (int64_t)(cells * copies) >= (1ll << 32)))
+      copies /= 2;
+    if (copies >= 8) break;
+    copies = 1;
+  }
+  if (copies == 1) list.clear();
+  std::fill(hot.begin(), hot.end(), 0u);
+  size_t at = (size_t)c->total_padded;
+  for (uint32_t sub : list) {
+    hot[sub] = (uint32_t)at;
+    at += (size_t)copies * c->h_sub[sub].padded_cells;
+  }
+  c->copies = copies;
+  c->tally_need = at;
+  return CMI_OK;
+}
+
+// the tally, zero between calls, grown to what the copies need
+int ensure_tally(cmi_context *c) {
+  if (!c->path || c->tally_need <= c->tally_words) return CMI_OK;
+  free_graph(c);
+  dev_free(c->d_tally);
+  c->tally_words = 0;
+  CMI_TRY(dev_alloc(&c->d_tally, c->tally_need));
+  c->tally_words = c->tally_need;
+  CMI_CUDA(cudaMemsetAsync(c->d_tally, 0, sizeof(unsigned long long) * c->tally_words, c->stream));
+  return CMI_OK;
+}
+
 // Upload instance + source tables (after sources or budgets change).
 int upload_tables(cmi_context *c) {
   bool reemission = false;
@@ -313,6 +448,9 @@ int upload_tables(cmi_context *c) {
     D.num_sources = (uint32_t)I.src_lum.size();
     D.num_cells = I.ncells;
     D.reemission = (float)I.reemission;
+    const float *csf = c->h_sub[I.first_sub].cell_size_f;
+    D.tally_weight =
+        (double)std::max(csf[0], std::max(csf[1], csf[2])) / 4194304.0 * I.desc.cross_section;
     const int32_t *ns = I.desc.num_subgrid;
     for (size_t k = 0; k < I.src_lum.size(); ++k) {
       DevSource s{};
@@ -352,6 +490,16 @@ int upload_tables(cmi_context *c) {
                              cudaMemcpyHostToDevice, c->stream));
   CMI_CUDA(cudaMemcpyAsync(c->d_inst, di.data(), sizeof(DevInstance) * di.size(),
                            cudaMemcpyHostToDevice, c->stream));
+  std::vector<DevGeo> geo;
+  std::vector<uint32_t> hot;
+  if (c->path) {
+    CMI_TRY(plan_tally_copies(c, hot));
+    CMI_CUDA(cudaMemcpyAsync(c->d_hot, hot.data(), sizeof(uint32_t) * hot.size(),
+                             cudaMemcpyHostToDevice, c->stream));
+    for (const HostInstance &I : c->inst) geo.push_back(instance_geometry(c, I));
+    CMI_CUDA(cudaMemcpyAsync(c->d_geo, geo.data(), sizeof(DevGeo) * geo.size(),
+                             cudaMemcpyHostToDevice, c->stream));
+  }
   CMI_CUDA(cudaStreamSynchronize(c->stream));
   free_graph(c);
   return CMI_OK;
@@ -573,6 +721,60 @@ int config_walk(cmi_context *c) {
   return config_kernel(c, k_walk64<kWalkThreads>);
 }
 
+template <class W, class WR, int kMin>
+int config_path_kernels(cmi_context *c) {
+  int per_sm[2] = {0, 0};  // without and with reemission
+  CMI_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm[0], k_path<W, false, kMin>,
+                                                         kPathThreads, c->path_smem));
+  CMI_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm[1], k_path<WR, true, kMin>,
+                                                         kPathThreads, c->path_smem));
+  for (int r = 0; r < 2; ++r) c->path_grid[r] = c->num_sms * std::max(per_sm[r], 1);
+  return CMI_OK;
+}
+// resident CTAs the builds of k_path are made for: registers against warps in flight
+// (B200, us per iteration at 5 / 6 / 7 CTAs: mixed, log-normal 128^3 2250 / 2036 / 2270;
+// FP64, 64^3 at 4 / 5 / 6 249 / 243 / 265; FP32, 96 x 80 x 112 at 7 / 8 / 9 707 / 718 / 779)
+constexpr int kPathMinM = 6, kPathMin32 = 8, kPathMin64 = 5;
+int config_path(cmi_context *c) {
+  if (!c->path) return CMI_OK;
+  if (c->fp32()) return config_path_kernels<Path32<true>, Path32<false>, kPathMin32>(c);
+  if (c->mixed()) return config_path_kernels<PathF<true, true>, PathF<true, false>, kPathMinM>(c);
+  return config_path_kernels<PathF<false, true>, PathF<false, false>, kPathMin64>(c);
+}
+
+template <class W, class WR, int kMin>
+void launch_path_t(cmi_context *c, const PathParams &p) {
+  if (c->reemission)
+    k_path<WR, true, kMin><<<c->path_grid[1], kPathThreads, c->path_smem, c->stream>>>(p);
+  else
+    k_path<W, false, kMin><<<c->path_grid[0], kPathThreads, c->path_smem, c->stream>>>(p);
+}
+int launch_path(cmi_context *c) {
+  PathParams p{};
+  p.geo = c->d_geo;
+  p.subs = c->d_sub;
+  p.inst = c->d_inst;
+  p.src = c->d_src;
+  p.nsrc_total = c->nsrc_total;
+  p.src_first = c->d_src_first;
+  p.st = c->d_state;
+  p.stats = c->d_stats;
+  p.kappa = c->d_kappa;
+  p.nH = c->d_nH;
+  p.xH = c->d_xH;
+  p.tally = c->d_tally;
+  p.hot = c->d_hot;
+  p.copies = c->copies;
+  p.table = c->path_table;
+  p.round_cap = (uint32_t)c->round_cap;
+  if (c->fp32()) launch_path_t<Path32<true>, Path32<false>, kPathMin32>(c, p);
+  else if (c->mixed()) launch_path_t<PathF<true, true>, PathF<true, false>, kPathMinM>(c, p);
+  else launch_path_t<PathF<false, true>, PathF<false, false>, kPathMin64>(c, p);
+  c->enqueued += 1;
+  CMI_CUDA(cudaGetLastError());
+  return CMI_OK;
+}
+
 EmitParams emit_params(cmi_context *c) {
   EmitParams e{};
   e.inst = c->d_inst;
@@ -656,17 +858,23 @@ int enqueue_rounds_graph(cmi_context *c) {
   return CMI_OK;
 }
 
+dim3 balance_grid(const cmi_context *c, uint32_t subgrids) {
+  return dim3(subgrids, (unsigned)((c->max_padded + kBalanceCells - 1) / kBalanceCells));
+}
+
 int enqueue_iteration(cmi_context *c, bool balance) {
   const int ninst = (int)c->inst.size();
   k_begin_iteration<<<1, 128, 0, c->stream>>>(c->d_state, c->d_stats, ninst);
   // Philox packets are written straight into their sorted place: the
   // emission plan fills the round-0 histogram, the plan places the buckets
   const bool direct = c->opt.rng == CMI_RNG_PHILOX;
+  const bool path = c->path;
   k_emission_plan<<<1, 128, 0, c->stream>>>(c->d_inst, ninst, c->d_src, c->nsrc_total,
                                             c->d_state, c->d_src_count, c->d_src_first,
                                             c->d_buf_first, c->d_stats,
-                                            direct ? c->d_src_rank0 : nullptr, c->d_hist);
+                                            direct && !path ? c->d_src_rank0 : nullptr, c->d_hist);
   c->enqueued += 2;
+  if (!path) {
   const EmitParams e = emit_params(c);
   const int egrid = c->num_sms * 8;
   if (direct) CMI_TRY(timed_launch(c, 1, [&] { return launch_plan(c, false); }));
@@ -685,12 +893,19 @@ int enqueue_iteration(cmi_context *c, bool balance) {
   c->enqueued += 1;
   CMI_CUDA(cudaGetLastError());
   if (!direct) CMI_TRY(timed_launch(c, 1, [&] { return launch_plan(c, true); }));
+  }
   // fields sent by cmi_set_fields_prefetched arrive on the copy stream: the
   // walk waits for them here, so their copy overlaps the emission above (a
   // graph holds this as an event-wait node on the latest record)
   CMI_CUDA(cudaStreamWaitEvent(c->stream, c->fields_ready,
                                c->capturing ? cudaEventWaitExternal : cudaEventWaitDefault));
-  CMI_TRY(c->capturing ? enqueue_rounds_graph(c) : enqueue_rounds(c));
+  if (path) CMI_TRY(timed_launch(c, 0, [&] { return launch_path(c); }));
+  else CMI_TRY(c->capturing ? enqueue_rounds_graph(c) : enqueue_rounds(c));
+  if (path && !balance) {
+    k_merge_tally<<<balance_grid(c, c->S), 256, 0, c->stream>>>(c->d_sub, c->d_inst, c->d_tally, c->d_hot,
+                                               c->copies, c->uses_kappa(), c->d_J);
+    c->enqueued += 1;
+  }
   if (balance) {
     BalanceParams b{};
     b.subs = c->d_sub;
@@ -703,11 +918,15 @@ int enqueue_iteration(cmi_context *c, bool balance) {
     b.first_sub = 0;
     b.num_subs = c->S;
     b.jfac_override = -1.;
+    b.tally = path ? c->d_tally : nullptr;
+    b.hot = c->d_hot;
+    b.copies = c->copies;
+    b.fixed = c->uses_kappa();
     CMI_TRY(timed_launch(c, 3, [&] {
       if (c->opt.balance_form == CMI_BALANCE_REFERENCE)
-        k_balance<0><<<c->S, 256, 0, c->stream>>>(b);
+        k_balance<0><<<balance_grid(c, c->S), 256, 0, c->stream>>>(b);
       else
-        k_balance<1><<<c->S, 256, 0, c->stream>>>(b);
+        k_balance<1><<<balance_grid(c, c->S), 256, 0, c->stream>>>(b);
       return CMI_OK;
     }));
     c->enqueued += 1;
@@ -718,12 +937,20 @@ int enqueue_iteration(cmi_context *c, bool balance) {
   return CMI_OK;
 }
 
+// memory of an iteration: arenas for its packets (wavefront), the tally (whole paths)
+int ensure_budget(cmi_context *c) {
+  const uint64_t n = total_budget(c);
+  if (!c->path) return ensure_capacity(c, n);
+  CMI_TRY(check_packets(n));
+  return ensure_tally(c);
+}
+
 int validate_ready(cmi_context *c) {
   for (size_t i = 0; i < c->inst.size(); ++i) {
     if (c->inst[i].num_photon > 0 && c->inst[i].src_lum.empty())
       return fail(CMI_ERR_INVALID_ARGUMENT, "instance %zu has a packet budget but no sources", i);
   }
-  return ensure_capacity(c, total_budget(c));
+  return ensure_budget(c);
 }
 
 void to_stats(const DevStats &d, const HostInstance &I, cmi_stats &s) {
@@ -797,7 +1024,7 @@ int run(cmi_context *c, int32_t iterations, uint64_t seed, uint32_t first_iterat
   CMI_CUDA(cudaStreamSynchronize(c->stream));
   uint32_t flags_any = 0;
   for (int32_t it = 0; it < iterations; ++it) {
-    if (use_graph && ninst > 0) {  // the round loop ran once per round with packets
+    if (use_graph && ninst > 0 && !c->path) {  // the round loop ran once per round with packets
       const uint32_t r = std::min<uint32_t>(c->h_stats[(size_t)it * ninst].rounds,
                                             (uint32_t)c->round_cap);
       c->last_launches += c->graph_body_kernels * r;
@@ -990,8 +1217,20 @@ int cmi_create(const cmi_grid_desc *grids, int32_t num_instances, const cmi_opti
   if (opt.packets_per_chunk == 0 && c->max_padded <= 1024) c->chunk = 256u;
   c->ntiles = (c->S + kPlanTile - 1) / kPlanTile;
 
+  // Transport by whole paths (cmi_path.cuh) unless something asks for the wavefront:
+  // the ranlxd replay (emission buffer by buffer), FP32 tallies, 2^31 cells or more,
+  // or subgrids so long that the face tables leave no room for six CTAs on an SM.
+  for (const auto &I : c->inst)
+    c->path_table = std::max(c->path_table, instance_geometry(c, I).table);
+  c->path_smem = (sizeof(PathShared) + sizeof(double) * (size_t)c->path_table) * kPathWarps;
+  c->path = opt.rng == CMI_RNG_PHILOX && c->total_padded < (1ll << 31) &&
+            c->path_smem <= kPathSmemMost &&
+            (c->fp64() || opt.tally_mode == CMI_TALLY_FIXED64 ||
+             opt.tally_mode == CMI_TALLY_FIXED64_ATOMIC64);
+
   int rc = CMI_OK;
-  if ((rc = dev_alloc(&c->d_sub, c->S)) || (rc = dev_alloc(&c->d_inst, c->inst.size())) ||
+  if ((rc = dev_alloc(&c->d_geo, c->inst.size())) || (rc = dev_alloc(&c->d_hot, c->S)) ||
+      (rc = dev_alloc(&c->d_sub, c->S)) || (rc = dev_alloc(&c->d_inst, c->inst.size())) ||
       (rc = dev_alloc(&c->d_nH, c->total_padded)) || (rc = dev_alloc(&c->d_xH, c->total_padded)) ||
       (rc = dev_alloc(&c->d_J, c->total_padded)) ||
       (rc = dev_alloc(&c->d_kappa, c->uses_kappa() ? c->total_padded : 1)) ||
@@ -1017,6 +1256,7 @@ int cmi_create(const cmi_grid_desc *grids, int32_t num_instances, const cmi_opti
   for (int32_t i = 0; i < num_instances; ++i)
     if ((rc = refresh_kappa(c, i))) return bail(rc);
   if ((rc = config_walk(c))) return bail(rc);
+  if ((rc = config_path(c))) return bail(rc);
   int64_t max_cells = 0;
   for (const auto &I : c->inst) max_cells = std::max(max_cells, I.ncells);
   if ((rc = ensure_stage(c, sizeof(double) * (size_t)max_cells))) return bail(rc);
@@ -1042,6 +1282,9 @@ int cmi_destroy(cmi_context *c) {
   dev_free(c->d_nH);
   dev_free(c->d_xH);
   dev_free(c->d_J);
+  dev_free(c->d_geo);
+  dev_free(c->d_tally);
+  dev_free(c->d_hot);
   dev_free(c->d_kappa);
   dev_free(c->d_src_count);
   dev_free(c->d_src_first);
@@ -1238,7 +1481,7 @@ int cmi_set_packet_budget(cmi_context *c, int32_t instance, uint64_t num_photon)
   CMI_TRY(check_instance(c, instance));
   c->inst[instance].num_photon = num_photon;
   CMI_TRY(upload_tables(c));
-  return ensure_capacity(c, total_budget(c));
+  return ensure_budget(c);
 }
 
 int cmi_set_reemission_probability(cmi_context *c, int32_t instance, double probability) {
@@ -1375,7 +1618,7 @@ int cmi_transport_packets(cmi_context *c, int32_t instance, const cmi_photon *pa
   if (n > 0 && (!packets || !start_subgrid))
     return fail(CMI_ERR_INVALID_ARGUMENT, "null packet arrays");
   CMI_TRY(clear_flags(c));
-  CMI_TRY(ensure_capacity(c, std::max<uint64_t>(n, total_budget(c))));
+  CMI_TRY(ensure_capacity(c, c->path ? n : std::max<uint64_t>(n, total_budget(c))));
   const size_t bytes = sizeof(Packet64) * n + sizeof(uint32_t) * n + 64;
   CMI_TRY(ensure_stage(c, bytes));
   Packet64 *d_ph = reinterpret_cast<Packet64 *>(c->d_stage);
@@ -1600,9 +1843,9 @@ int cmi_compute_neutral_fraction_subgrids(cmi_context *c, int32_t instance,
   b.num_subs = count;
   b.jfac_override = jfac;
   if (c->opt.balance_form == CMI_BALANCE_REFERENCE)
-    k_balance<0><<<count, 256, 0, c->stream>>>(b);
+    k_balance<0><<<balance_grid(c, count), 256, 0, c->stream>>>(b);
   else
-    k_balance<1><<<count, 256, 0, c->stream>>>(b);
+    k_balance<1><<<balance_grid(c, count), 256, 0, c->stream>>>(b);
   CMI_CUDA(cudaGetLastError());
   DevStats d{};
   CMI_CUDA(cudaMemcpyAsync(&d, c->d_stats + instance, sizeof(DevStats), cudaMemcpyDeviceToHost,

@@ -139,6 +139,7 @@ __global__ void k_begin_iteration(RoundState *st, DevStats *stats, int ninst) {
     st->chunk_next = 0;
     st->total_in = 0;
   }
+  if (threadIdx.x < kPathShares) st->share_next[threadIdx.x] = 0;
 }
 
 __global__ void k_end_iteration(RoundState *st, DevStats *stats, int ninst, int advance) {
@@ -1519,8 +1520,36 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_walkm(WalkParams prm) 
 }
 
 // ---------------------------------------------------------------------------
-// ionization balance (DensitySubGrid.hpp:1628-1658), one block per subgrid
+// ionization balance (DensitySubGrid.hpp:1628-1658), blocks of kBalanceCells cells of a
+// subgrid (grid: subgrids x blocks of the largest)
 // ---------------------------------------------------------------------------
+// Tally of cell c of a subgrid (with its copies), reset: the path lengths of the
+// transport in units of J.
+__device__ __forceinline__ double take_tally(unsigned long long *tally, int64_t i, uint32_t hot,
+                                             uint32_t copies, uint32_t padded, int c, bool fixed,
+                                             const DevInstance &I) {
+  unsigned long long t = tally[i];
+  double d = fixed ? 0. : __longlong_as_double((long long)t);
+  if (t) tally[i] = 0ull;
+  if (hot) {
+    unsigned long long *q = tally + hot + c;
+    for (uint32_t r = 0; r < copies; r += 8) {  // eight loads on the way (copies: of 8)
+      unsigned long long v[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v[k] = q[(size_t)(r + k) * padded];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        if (!v[k]) continue;
+        if (fixed) t += v[k]; else d += __longlong_as_double((long long)v[k]);
+        q[(size_t)(r + k) * padded] = 0ull;
+      }
+    }
+  }
+  return fixed ? (double)t * I.tally_weight : d;
+}
+
+constexpr int kBalanceCells = 512;  // cells of a subgrid per block
+
 struct BalanceParams {
   const DevSubgrid *subs;
   const DevInstance *inst;
@@ -1530,6 +1559,10 @@ struct BalanceParams {
   DevStats *stats;
   uint32_t first_sub, num_subs;
   double jfac_override;  // >= 0: use instead of the instance's jfac
+  unsigned long long *tally;  // of the path kernel, added to J and reset (may be null)
+  const uint32_t *hot;
+  uint32_t copies;
+  bool fixed;
 };
 
 template <int kForm>
@@ -1543,9 +1576,14 @@ __global__ void __launch_bounds__(256) k_balance(BalanceParams prm) {
   const double alpha = I.alpha;
   const double sigma = I.sigma;
   double dx = 0.;
-  for (int c = threadIdx.x; c < S.ncells; c += blockDim.x) {
+  const int end = min(S.ncells, (int)(blockIdx.y + 1) * kBalanceCells);
+  for (int c = (int)blockIdx.y * kBalanceCells + threadIdx.x; c < end; c += blockDim.x) {
     const int64_t i = S.field_offset + c;
-    const double jH = jfac * prm.J[i];
+    double J = prm.J[i];
+    if (prm.tally)
+      J += take_tally(prm.tally, i, prm.hot[s], prm.copies, (uint32_t)S.padded_cells, c, prm.fixed,
+                      I);
+    const double jH = jfac * J;
     const double x_old = prm.xH[i];
     double x;
     if (jH > 0.) {
