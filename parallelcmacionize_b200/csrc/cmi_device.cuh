@@ -292,6 +292,21 @@ __device__ __forceinline__ uint32_t reemit_hash(double x) {
   return (uint32_t)b ^ (uint32_t)(b >> 32);
 }
 
+// a / n for a small integer n, correctly rounded: with y = 1 / n rounded, q = a y is
+// within an ulp and q + (a - n q) y rounds correctly (Markstein, IBM J. Res. Dev. 34,
+// 1990; the residual is exact by the fused multiply-add).  Three operations instead of
+// a division; below the normal range it may be off, which the series here never add
+// to a visible sum.
+__host__ __device__ __forceinline__ double over_integer(double a, int n) {
+#ifdef __CUDA_ARCH__
+  const double y = 1.0 / (double)n;  // of a constant where the loop is unrolled
+  const double q = __dmul_rn(a, y);
+  return __fma_rn(__fma_rn(-(double)n, q, a), y, q);
+#else
+  return a / (double)n;
+#endif
+}
+
 // -ln(u) for u in (0, 1): u = m 2^e with m in [sqrt(1/2), sqrt(2)), then
 // ln m = 2 (s + s^3/3 + ... + s^31/31), s = (m - 1) / (m + 1), |s| < 0.1716
 __device__ __forceinline__ double reemit_neg_log(double u) {
@@ -304,9 +319,10 @@ __device__ __forceinline__ double reemit_neg_log(double u) {
   const double s = (m - 1.) / (m + 1.);
   const double s2 = s * s;
   double term = s, sum = s;
+#pragma unroll
   for (int k = 3; k <= 31; k += 2) {
     term *= s2;
-    sum += term / (double)k;
+    sum += over_integer(term, k);
   }
   return -(2. * sum + (double)e * 0.69314718055994530942);
 }

@@ -51,8 +51,11 @@ __host__ __device__ inline double dust_exp(double x) {
   const double k = rint(x * 0x1.71547652b82fep+0);
   const double r = (x - k * 0x1.62e42fefa3800p-1) - k * 0x1.ef35793c76730p-45;
   double term = 1., sum = 1.;
+#ifdef __CUDA_ARCH__
+#pragma unroll
+#endif
   for (int n = 1; n <= 18; ++n) {
-    term = term * r / (double)n;
+    term = over_integer(term * r, n);
     sum += term;
   }
   return ldexp(sum, (int)k);
@@ -74,9 +77,12 @@ __host__ __device__ inline double dust_neg_log(double u) {
   const double s = (m - 1.) / (m + 1.);
   const double s2 = s * s;
   double term = s, sum = s;
+#ifdef __CUDA_ARCH__
+#pragma unroll
+#endif
   for (int k = 3; k <= 31; k += 2) {
     term *= s2;
-    sum += term / (double)k;
+    sum += over_integer(term, k);
   }
   return -(2. * sum + (double)e * 0.69314718055994530942);
 }

@@ -6,6 +6,7 @@
 #include "cmi_kernels.cuh"
 #include "cmi_dust.cuh"
 #include "cmi_path.cuh"
+#include "cmi_dust_path.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -143,6 +144,7 @@ struct cmi_context {
 
   // whole-path transport (cmi_path.cuh) instead of the wavefront, and what it needs
   bool path = false;
+  bool tables_fit = false;  // path_table fits, whatever carries the iterations
   DevGeo *d_geo = nullptr;
   unsigned long long *d_tally = nullptr;
   uint32_t *d_hot = nullptr;   // per subgrid: first cell of its tally copies, 0: none
@@ -496,6 +498,8 @@ int upload_tables(cmi_context *c) {
     CMI_TRY(plan_tally_copies(c, hot));
     CMI_CUDA(cudaMemcpyAsync(c->d_hot, hot.data(), sizeof(uint32_t) * hot.size(),
                              cudaMemcpyHostToDevice, c->stream));
+  }
+  if (c->tables_fit) {
     for (const HostInstance &I : c->inst) geo.push_back(instance_geometry(c, I));
     CMI_CUDA(cudaMemcpyAsync(c->d_geo, geo.data(), sizeof(DevGeo) * geo.size(),
                              cudaMemcpyHostToDevice, c->stream));
@@ -1223,8 +1227,8 @@ int cmi_create(const cmi_grid_desc *grids, int32_t num_instances, const cmi_opti
   for (const auto &I : c->inst)
     c->path_table = std::max(c->path_table, instance_geometry(c, I).table);
   c->path_smem = (sizeof(PathShared) + sizeof(double) * (size_t)c->path_table) * kPathWarps;
-  c->path = opt.rng == CMI_RNG_PHILOX && c->total_padded < (1ll << 31) &&
-            c->path_smem <= kPathSmemMost &&
+  c->tables_fit = c->total_padded < (1ll << 31) && c->path_smem <= kPathSmemMost;
+  c->path = c->tables_fit && opt.rng == CMI_RNG_PHILOX &&
             (c->fp64() || opt.tally_mode == CMI_TALLY_FIXED64 ||
              opt.tally_mode == CMI_TALLY_FIXED64_ATOMIC64);
 
@@ -1957,6 +1961,81 @@ void free_dust_buffers(DustBuffers *b) { delete b; }
 
 namespace {
 
+// image and statistics of a dust run
+int dust_result(cmi_context *c, uint64_t num_photon, size_t npix, const double *d_image,
+                const unsigned long long *d_counters, uint32_t generations, double *image,
+                cmi_dust_stats *stats) {
+  unsigned long long ctr[8];
+  CMI_CUDA(cudaMemcpyAsync(image, d_image, sizeof(double) * npix, cudaMemcpyDeviceToHost,
+                           c->stream));
+  CMI_CUDA(cudaMemcpyAsync(ctr, d_counters, sizeof(ctr), cudaMemcpyDeviceToHost, c->stream));
+  CMI_CUDA(cudaStreamSynchronize(c->stream));
+  // the driver's image.dat holds the sums divided by the packet count
+  for (size_t k = 0; k < npix; ++k) image[k] /= (double)num_photon;
+  if (stats) {
+    std::memset(stats, 0, sizeof(*stats));
+    stats->emitted = num_photon;
+    stats->cell_crossings = ctr[0];
+    stats->subgrid_transits = ctr[1];
+    stats->absorbed = ctr[3];
+    stats->escaped = ctr[4];
+    stats->scatterings = ctr[5];
+    stats->peeloffs_off_image = ctr[6];
+    // passes of walk + scatter: one more than the scatterings of any packet
+    stats->generations = generations ? generations
+                                     : std::min<uint32_t>((uint32_t)ctr[7] + 1u, kDustMaxGenerations);
+    stats->error_flags = ctr[2] ? (uint32_t)kFlagWalkLimit : 0u;
+  }
+  if (ctr[2]) return fail(CMI_ERR_INVARIANT, "dust walk: step or visit bound exceeded");
+  return CMI_OK;
+}
+
+constexpr int kDustPathMin = 5;  // resident CTAs k_dust_path is built for (6: 10.5 for 10.0 ms)
+
+int dust_by_paths(cmi_context *c, int32_t instance, uint32_t n, uint64_t seed, uint32_t iteration,
+                  double albedo, const double source[3], uint32_t src_sub, int32_t npix_x,
+                  int32_t npix_y, double *image, cmi_dust_stats *stats) {
+  const size_t npix = (size_t)npix_x * npix_y;
+  // counters, claims, then the image
+  const size_t head = 16;  // doubles
+  CMI_TRY(ensure_stage(c, sizeof(double) * (npix + head)));
+  CMI_CUDA(cudaMemsetAsync(c->d_stage, 0, sizeof(double) * (npix + head), c->stream));
+  DustPathParams p{};
+  p.path.geo = c->d_geo + instance;
+  p.path.subs = c->d_sub;
+  p.path.nH = c->d_nH;
+  p.path.xH = c->d_xH;
+  p.path.table = c->path_table;
+  p.n = n;
+  p.counters = reinterpret_cast<unsigned long long *>(c->d_stage);
+  p.next = reinterpret_cast<uint32_t *>(c->d_stage + 8);
+  p.image = c->d_stage + head;
+  p.seed = seed;
+  p.instance = (uint32_t)instance;
+  p.iteration = iteration;
+  p.src_sub = src_sub;
+  for (int a = 0; a < 3; ++a) p.src[a] = source[a];
+  p.albedo = albedo;
+  const double *box = c->inst[instance].desc.box;
+  p.x0 = box[0];
+  p.wx = box[3];
+  p.y0 = box[1];
+  p.wy = box[4];
+  p.npx = npix_x;
+  p.npy = npix_y;
+  const size_t smem = (sizeof(PathShared) + sizeof(DustLanes) +
+                       sizeof(double) * (size_t)c->path_table) * kPathWarps;
+  static_assert(kPathSmemMost + sizeof(DustLanes) * kPathWarps <= 49152, "no opt-in needed");
+  int per_sm = 0;
+  CMI_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_dust_path<kDustPathMin>,
+                                                         kPathThreads, smem));
+  const int grid = std::max(1, std::min<int>(c->num_sms * std::max(per_sm, 1),
+                                             (int)((n + kPathThreads - 1) / kPathThreads)));
+  k_dust_path<kDustPathMin><<<grid, kPathThreads, smem, c->stream>>>(p);
+  CMI_CUDA(cudaGetLastError());
+  return dust_result(c, n, npix, p.image, p.counters, 0u, image, stats);
+}
+
 unsigned dust_blocks(uint64_t n, int threads) {
   return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((n + threads - 1) / threads, 148 * 32));
 }
@@ -2037,6 +2116,11 @@ extern "C" int cmi_dust_run(cmi_context *c, int32_t instance, uint64_t num_photo
   }
   const uint32_t n = (uint32_t)num_photon;
   const size_t npix = (size_t)npix_x * npix_y;
+  const uint32_t src_sub =
+      (uint32_t)((si[0] * I.desc.num_subgrid[1] + si[1]) * I.desc.num_subgrid[2] + si[2]);
+  if (c->tables_fit)
+    return dust_by_paths(c, instance, n, seed, iteration, albedo, source, src_sub, npix_x, npix_y,
+                         image, stats);
   // the buffers grow to the largest call and stay with the context (about
   // 290 bytes per packet); a failed allocation leaves no buffers behind
   if (!c->dust || c->dust_capacity < n || c->dust_pixels < npix) {
@@ -2087,8 +2171,7 @@ extern "C" int cmi_dust_run(cmi_context *c, int32_t instance, uint64_t num_photo
   p.instance = (uint32_t)instance;
   p.iteration = iteration;
   for (int a = 0; a < 3; ++a) p.src[a] = source[a];
-  p.src_sub = I.first_sub + (uint32_t)((si[0] * I.desc.num_subgrid[1] + si[1]) *
-                                           I.desc.num_subgrid[2] + si[2]);
+  p.src_sub = I.first_sub + src_sub;
   p.counters = B.counters;
   auto pass = [&](int k) {
     p.pk = B.pk[k];
@@ -2152,27 +2235,7 @@ extern "C" int cmi_dust_run(cmi_context *c, int32_t instance, uint64_t num_photo
     CMI_CUDA(cudaGetLastError());
     cur = 1 - cur;
   }
-  std::vector<double> img(npix);
-  unsigned long long ctr[8];
-  CMI_CUDA(cudaMemcpyAsync(img.data(), B.image, sizeof(double) * npix, cudaMemcpyDeviceToHost, st));
-  CMI_CUDA(cudaMemcpyAsync(ctr, B.counters, sizeof(ctr), cudaMemcpyDeviceToHost, st));
-  CMI_CUDA(cudaStreamSynchronize(st));
-  // the driver's image.dat holds the sums divided by the packet count
-  for (size_t k = 0; k < npix; ++k) image[k] = img[k] / (double)num_photon;
-  if (stats) {
-    std::memset(stats, 0, sizeof(*stats));
-    stats->emitted = num_photon;
-    stats->cell_crossings = ctr[0];
-    stats->subgrid_transits = ctr[1];
-    stats->absorbed = ctr[3];
-    stats->escaped = ctr[4];
-    stats->scatterings = ctr[5];
-    stats->peeloffs_off_image = ctr[6];
-    stats->generations = generations;
-    stats->error_flags = ctr[2] ? (uint32_t)kFlagWalkLimit : 0u;
-  }
-  if (ctr[2]) return fail(CMI_ERR_INVARIANT, "dust walk: step or visit bound exceeded");
-  return CMI_OK;
+  return dust_result(c, num_photon, npix, B.image, B.counters, generations, image, stats);
 }
 
 // ===========================================================================

@@ -193,7 +193,7 @@ __device__ __forceinline__ uint32_t exit_sides(uint32_t out, const float sg[3]) 
 // WalkM / Walk64, with the cell as an index into the whole field and the face
 // ahead read from the instance's table; the entry beyond the last face is a
 // guard whose high word marks the exit.
-template <bool kMixed, bool kDefer>
+template <bool kMixed, bool kDefer, bool kTally = true>
 struct PathF {
   using Real = typename std::conditional<kMixed, float, double>::type;
   double pos[3], d[3], inv[3], face[3];
@@ -206,7 +206,8 @@ struct PathF {
   Real done, target;
   int steps;
   uint32_t ex;          // exit: bit a axis a, bit 3 + a through the high face
-  // kDefer: the last crossing, its opacity (FP64: n_H, x_H) still on the way
+  // kDefer: the last crossing, its opacity (FP64: n_H, x_H) still on the way; else the
+  // opacity of the present cell
   double last;
   Real lk, lx;
   uint32_t lat;
@@ -264,17 +265,22 @@ struct PathF {
     if (out) return kExited;
     cell = g.first_cell + sub * g.padded +
            (uint32_t)(idx[0] * g.stride[0] + idx[1] * g.stride[1] + idx[2]);
-    toff = tally_offset(prm, g, sub, copy);
+    toff = kTally ? tally_offset(prm, g, sub, copy) : 0u;
 #pragma unroll
     for (int a = 0; a < 3; ++a) ahead(g, tab, a, idx[a]);
+    if (!kDefer) opacity(prm, lk, lx);
     return kRun;
   }
 
   // the state of a packet at the source, shared by the warp
   __device__ __forceinline__ void at_source(const PathParams &prm, uint32_t copy, PathShared &sh,
                                             uint32_t tab, const DevSource &S) {
+    at_position(prm, copy, sh, tab, S.position, S.subgrid - sh.geo.first_sub);
+  }
+  __device__ __forceinline__ void at_position(const PathParams &prm, uint32_t copy,
+                                              PathShared &sh, uint32_t tab,
+                                              const double position[3], uint32_t sub) {
     const DevGeo &g = sh.geo;
-    const uint32_t sub = S.subgrid - g.first_sub;
     int idx[3];
     double anchor[3];
     for (int a = 0; a < 3; ++a) {
@@ -282,7 +288,7 @@ struct PathF {
                                           (int)(sub / (uint32_t)g.sub_stride[a]) % g.ns[a]);
       anchor[a] = table_at(sh.src_c[a]);
     }
-    const uint32_t out = locate(g, anchor, S.position, 0u, idx);
+    const uint32_t out = locate(g, anchor, position, 0u, idx);
     for (int a = 0; a < 3; ++a) {
       sh.src_pos[a] = pos[a];
       sh.src_idx[a] = idx[a];
@@ -290,10 +296,11 @@ struct PathF {
     sh.src_sub = sub;
     sh.src_cell = g.first_cell + sub * g.padded +
                   (uint32_t)(idx[0] * g.stride[0] + idx[1] * g.stride[1] + idx[2]);
-    sh.src_toff = tally_offset(prm, g, sub, copy);
+    sh.src_toff = kTally ? tally_offset(prm, g, sub, copy) : 0u;
     sh.src_out = out;
   }
-  __device__ __forceinline__ int start(PathShared &sh, int lane, uint32_t tab) {
+  __device__ __forceinline__ int start(const PathParams &prm, PathShared &sh, int lane,
+                                       uint32_t tab) {
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
       pos[a] = sh.src_pos[a];
@@ -305,7 +312,9 @@ struct PathF {
     toff = sh.src_toff;
     if (!((Real)0 < target)) return kAbsorbed;
     ex = sh.src_out;
-    return ex ? kExited : kRun;
+    if (ex) return kExited;
+    if (!kDefer) opacity(prm, lk, lx);
+    return kRun;
   }
 
   // Entry into the subgrid on the other side of the faces in `in` (bit a: axis a, bit
@@ -376,10 +385,11 @@ struct PathF {
     if (outside) return kPathFree;
     sh.sub[lane] = sub;
     if (same) {
-      toff = tally_offset(prm, g, sub, copy);
+      if (kTally) toff = tally_offset(prm, g, sub, copy);
       // the guard on the axes it left by: read again
 #pragma unroll
       for (int a = 0; a < 3; ++a) face[a] = table_at(fi[a]);
+      if (!kDefer) opacity(prm, lk, lx);
       return (Real)0 < target ? kRun : kAbsorbed;
     }
     uint32_t in = 0;
@@ -420,13 +430,13 @@ struct PathF {
       const float lf = __double2float_rn(lmin);
       const Real after = (Real)__fadd_rn((float)done, __fmul_rn(lf, (float)k));
       if (after >= target) return false;
-      add_tally(prm.tally + at, Tally32<3>::fixed(lf, scale));
+      if (kTally) add_tally(prm.tally + at, Tally32<3>::fixed(lf, scale));
       done = after;
     } else {
       const double ls = __dmul_rn(lmin, g.sigma);
       const Real after = (Real)__dadd_rn((double)done, __dmul_rn(__dmul_rn(ls, (double)k), (double)x));
       if (after >= target) return false;
-      add_tally(prm.tally + at, ls);
+      if (kTally) add_tally(prm.tally + at, ls);
       done = after;
     }
     return true;
@@ -438,13 +448,14 @@ struct PathF {
       const float tau = __fmul_rn(__double2float_rn(lmin), (float)k);
       const float frac = fminf(__fdiv_rn(__fsub_rn((float)target, (float)done), tau), 1.f);
       lmin = __dmul_rn(lmin, (double)frac);
-      add_tally(prm.tally + at, Tally32<3>::fixed(__double2float_rn(lmin), scale));
+      if (kTally)
+        add_tally(prm.tally + at, Tally32<3>::fixed(__double2float_rn(lmin), scale));
     } else {
       const double tau = __dmul_rn(__dmul_rn(__dmul_rn(lmin, g.sigma), (double)k), (double)x);
       const double after = __dadd_rn((double)done, tau);
       const double correction = __ddiv_rn(__dsub_rn(after, (double)target), tau);
       lmin = __dmul_rn(lmin, __dsub_rn(1., correction));
-      add_tally(prm.tally + at, __dmul_rn(lmin, g.sigma));
+      if (kTally) add_tally(prm.tally + at, __dmul_rn(lmin, g.sigma));
     }
     return lmin;
   }
@@ -465,7 +476,7 @@ struct PathF {
   // load has had a whole turn to come back.
   __device__ __forceinline__ int step(const PathParams &prm, const DevGeo &g, uint32_t tab) {
     Real k, x;
-    opacity(prm, k, x);
+    if (kDefer) opacity(prm, k, x);
     double l[3];
 #pragma unroll
     for (int a = 0; a < 3; ++a) l[a] = __dmul_rn(__dsub_rn(face[a], pos[a]), inv[a]);
@@ -477,7 +488,7 @@ struct PathF {
       lx = x;
       lat = cell + toff;
     } else {
-      if (!pass(prm, g, lmin, k, x, cell + toff)) return kAbsorbed;
+      if (!pass(prm, g, lmin, lk, lx, cell + toff)) return kAbsorbed;
     }
     ++steps;
 #pragma unroll
@@ -489,7 +500,9 @@ struct PathF {
     // faces are not negative, so their high words order like integers
     const int top = max(__double2hiint(face[0]),
                         max(__double2hiint(face[1]), __double2hiint(face[2])));
-    return top >= (int)kGuardHi ? kExited : kRun;
+    if (top >= (int)kGuardHi) return kExited;
+    if (!kDefer) opacity(prm, lk, lx);
+    return kRun;
   }
 
   // at a subgrid face: the depth of the crossing that led there
@@ -511,9 +524,7 @@ struct PathF {
       double l[3];
 #pragma unroll
       for (int a = 0; a < 3; ++a) l[a] = __dmul_rn(__dsub_rn(face[a], pos[a]), inv[a]);
-      Real k, x;
-      opacity(prm, k, x);
-      const double lmin = stop(prm, g, min_ref(l[0], min_ref(l[1], l[2])), k, x, cell + toff);
+      const double lmin = stop(prm, g, min_ref(l[0], min_ref(l[1], l[2])), lk, lx, cell + toff);
       ++steps;
       if (kReemit) {
 #pragma unroll
@@ -610,7 +621,7 @@ struct Path32 {
     sh.src_toff = tally_offset(prm, g, sub, copy);
     sh.src_out = out;
   }
-  __device__ __forceinline__ int start(PathShared &sh, int lane, uint32_t) {
+  __device__ __forceinline__ int start(const PathParams &, PathShared &sh, int lane, uint32_t) {
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
       p[a] = (float)sh.src_pos[a];
@@ -925,7 +936,7 @@ __global__ void __launch_bounds__(kPathThreads, kMinBlocks) k_path(const __grid_
         if (status == kPathFree && r < q_n) {
           for (int a = 0; a < 3; ++a) w.direction(sh.geo, a, sh.q_dir[a][r], sh.q_inv[a][r]);
           w.depth(sh.q_tau[r]);
-          status = w.start(sh, lane, tab);
+          status = w.start(prm, sh, lane, tab);
           sh.visits[lane] = 1u;
           if (kReemit) sh.again[lane] = 0u;
         }
