@@ -139,8 +139,17 @@ struct alignas(16) RoundState {
   uint32_t rounds_active;
   uint32_t capacity;       // arena capacity (packets)
   uint32_t round_index;    // walks started this iteration (graph loop)
-  uint32_t pad[2];
+  uint32_t ticket;         // RunArgs taken
+  uint32_t slot;           // iterations of the call finished
+  uint32_t blocks_done;    // of the balance, back to 0 when all are
   uint32_t share_next[kPathShares];  // packets claimed of each share (path kernel)
+};
+
+// What a run passes to its first iteration, in pinned host memory.
+struct RunArgs {
+  uint64_t seed;
+  uint32_t iteration;
+  uint32_t ticket;         // another one for every call
 };
 
 // FP64 packet: the reference Photon layout (80 B); `meta` (the reserved

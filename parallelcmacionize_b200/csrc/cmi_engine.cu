@@ -169,7 +169,12 @@ struct cmi_context {
   uint64_t graph_body_kernels = 0;  // kernels per round of the loop
   uint64_t last_launches = 0;
   uint64_t enqueued = 0;  // kernel launches of the current enqueue
-  DevStats *h_stats = nullptr;  // pinned
+  DevStats *h_stats = nullptr;  // pinned; the iterations of a call write theirs in order
+  RunArgs *h_args = nullptr;    // pinned
+  char *h_pin = nullptr;        // pinned: small copies of cmi_traverse_buffer, cmi_trace_packet
+  size_t h_pin_bytes = 0;
+  bool traverse_ready = false;  // k_traverse's shared-memory limit set
+  uint32_t iteration = 0;       // index of the next iteration (the device counts along)
   size_t h_stats_count = 0;
 
   // optional per-kernel event timing
@@ -868,16 +873,15 @@ dim3 balance_grid(const cmi_context *c, uint32_t subgrids) {
 
 int enqueue_iteration(cmi_context *c, bool balance) {
   const int ninst = (int)c->inst.size();
-  k_begin_iteration<<<1, 128, 0, c->stream>>>(c->d_state, c->d_stats, ninst);
   // Philox packets are written straight into their sorted place: the
   // emission plan fills the round-0 histogram, the plan places the buckets
   const bool direct = c->opt.rng == CMI_RNG_PHILOX;
   const bool path = c->path;
-  k_emission_plan<<<1, 128, 0, c->stream>>>(c->d_inst, ninst, c->d_src, c->nsrc_total,
-                                            c->d_state, c->d_src_count, c->d_src_first,
-                                            c->d_buf_first, c->d_stats,
-                                            direct && !path ? c->d_src_rank0 : nullptr, c->d_hist);
-  c->enqueued += 2;
+  k_begin_emission<<<1, kBeginThreads, 0, c->stream>>>(
+      c->d_inst, ninst, c->d_src, c->nsrc_total, c->d_state, c->d_src_count, c->d_src_first,
+      c->d_buf_first, c->d_stats, direct && !path ? c->d_src_rank0 : nullptr, c->d_hist,
+      c->h_args, path ? (uint32_t)c->path_grid[c->reemission ? 1 : 0] : 0u);
+  c->enqueued += 1;
   if (!path) {
   const EmitParams e = emit_params(c);
   const int egrid = c->num_sms * 8;
@@ -926,6 +930,9 @@ int enqueue_iteration(cmi_context *c, bool balance) {
     b.hot = c->d_hot;
     b.copies = c->copies;
     b.fixed = c->uses_kappa();
+    b.st = c->d_state;
+    b.ninst = ninst;
+    b.host = c->h_stats;
     CMI_TRY(timed_launch(c, 3, [&] {
       if (c->opt.balance_form == CMI_BALANCE_REFERENCE)
         k_balance<0><<<balance_grid(c, c->S), 256, 0, c->stream>>>(b);
@@ -935,8 +942,10 @@ int enqueue_iteration(cmi_context *c, bool balance) {
     }));
     c->enqueued += 1;
   }
-  k_end_iteration<<<1, 128, 0, c->stream>>>(c->d_state, c->d_stats, ninst, 1);
-  c->enqueued += 1;
+  if (!balance) {
+    k_end_iteration<<<1, 128, 0, c->stream>>>(c->d_state, c->d_stats, ninst, 1, c->h_stats);
+    c->enqueued += 1;
+  }
   CMI_CUDA(cudaGetLastError());
   return CMI_OK;
 }
@@ -971,8 +980,10 @@ void to_stats(const DevStats &d, const HostInstance &I, cmi_stats &s) {
 
 int ensure_host_stats(cmi_context *c, size_t n) {
   if (n <= c->h_stats_count) return CMI_OK;
+  free_graph(c);  // its last kernel writes there
   if (c->h_stats) cudaFreeHost(c->h_stats);
   c->h_stats = nullptr;
+  c->h_stats_count = 0;
   CMI_CUDA(cudaMallocHost((void **)&c->h_stats, sizeof(DevStats) * n));
   c->h_stats_count = n;
   return CMI_OK;
@@ -983,11 +994,11 @@ int run(cmi_context *c, int32_t iterations, uint64_t seed, uint32_t first_iterat
   CMI_TRY(validate_ready(c));
   const int ninst = (int)c->inst.size();
   CMI_TRY(ensure_host_stats(c, (size_t)iterations * ninst));
-  const uint64_t hs[2] = {seed, 0};
-  CMI_CUDA(cudaMemcpyAsync(&c->d_state->seed, hs, sizeof(uint64_t), cudaMemcpyHostToDevice,
-                           c->stream));
-  CMI_CUDA(cudaMemcpyAsync(&c->d_state->iteration, &first_iteration, sizeof(uint32_t),
-                           cudaMemcpyHostToDevice, c->stream));
+  // the first kernel takes these up and clears the flags; nothing of an earlier call
+  // is in flight (every call waits for its iterations)
+  c->h_args->seed = seed;
+  c->h_args->iteration = first_iteration;
+  c->h_args->ticket += 1u;
   c->last_launches = 0;
   const bool use_graph = c->opt.use_graph != 0 && !c->timing;
   const int gi = balance ? 1 : 0;
@@ -1021,8 +1032,7 @@ int run(cmi_context *c, int32_t iterations, uint64_t seed, uint32_t first_iterat
       CMI_TRY(enqueue_iteration(c, balance));
       c->last_launches += c->enqueued;
     }
-    CMI_CUDA(cudaMemcpyAsync(c->h_stats + (size_t)it * ninst, c->d_stats,
-                             sizeof(DevStats) * ninst, cudaMemcpyDeviceToHost, c->stream));
+    c->iteration = first_iteration + (uint32_t)it + 1u;
     c->fields_pending = false;  // the iteration waited for the fields
   }
   CMI_CUDA(cudaStreamSynchronize(c->stream));
@@ -1267,6 +1277,9 @@ int cmi_create(const cmi_grid_desc *grids, int32_t num_instances, const cmi_opti
   if ((rc = ensure_capacity(c, 1024))) return bail(rc);
   // pinned per-iteration statistics: allocated here, not inside a timed run
   if ((rc = ensure_host_stats(c, 256 * c->inst.size()))) return bail(rc);
+  if (cudaMallocHost((void **)&c->h_args, sizeof(RunArgs)) != cudaSuccess)
+    return bail(fail(CMI_ERR_OUT_OF_MEMORY, "pinned allocation failed"));
+  std::memset(c->h_args, 0, sizeof(RunArgs));
   if (cudaStreamSynchronize(c->stream) != cudaSuccess)
     return bail(fail(CMI_ERR_CUDA, "context set-up failed: %s",
                      cudaGetErrorString(cudaGetLastError())));
@@ -1312,6 +1325,8 @@ int cmi_destroy(cmi_context *c) {
   free_dust_buffers(c->dust);
   c->dust = nullptr;
   if (c->h_stats) cudaFreeHost(c->h_stats);
+  if (c->h_args) cudaFreeHost(c->h_args);
+  if (c->h_pin) cudaFreeHost(c->h_pin);
   for (auto &t : c->timed) {
     cudaEventDestroy(t.start);
     cudaEventDestroy(t.stop);
@@ -1500,13 +1515,8 @@ int cmi_set_reemission_probability(cmi_context *c, int32_t instance, double prob
 int cmi_run_iterations(cmi_context *c, int32_t iterations, uint64_t seed, cmi_stats *stats) {
   CMI_TRY(check_ctx(c, false));
   if (iterations <= 0) return fail(CMI_ERR_INVALID_ARGUMENT, "iterations must be > 0");
-  CMI_TRY(clear_flags(c));
   // the first iteration index of this call continues from the previous call
-  uint32_t it0 = 0;
-  CMI_CUDA(cudaMemcpyAsync(&it0, &c->d_state->iteration, sizeof(uint32_t), cudaMemcpyDeviceToHost,
-                           c->stream));
-  CMI_CUDA(cudaStreamSynchronize(c->stream));
-  return run(c, iterations, seed, it0, true, stats);
+  return run(c, iterations, seed, c->iteration, true, stats);
 }
 
 static int set_frozen(cmi_context *c, int32_t i, uint32_t v) {
@@ -1527,11 +1537,7 @@ int cmi_run_until_converged(cmi_context *c, int32_t max_iterations, int32_t min_
   const int ninst = (int)c->inst.size();
   std::vector<int32_t> at(ninst, 0);
   int remaining = ninst;
-  CMI_TRY(clear_flags(c));
-  uint32_t it0 = 0;
-  CMI_CUDA(cudaMemcpyAsync(&it0, &c->d_state->iteration, sizeof(uint32_t), cudaMemcpyDeviceToHost,
-                           c->stream));
-  CMI_CUDA(cudaStreamSynchronize(c->stream));
+  const uint32_t it0 = c->iteration;
   std::vector<cmi_stats> st(ninst);
   int32_t done = 0;
   int rc = CMI_OK;
@@ -1582,10 +1588,10 @@ int cmi_emit_photons(cmi_context *c, uint64_t seed, uint32_t iteration, cmi_phot
   CMI_CUDA(cudaMemcpyAsync(&c->d_state->iteration, &iteration, sizeof(uint32_t),
                            cudaMemcpyHostToDevice, c->stream));
   const int ninst = (int)c->inst.size();
-  k_begin_iteration<<<1, 128, 0, c->stream>>>(c->d_state, c->d_stats, ninst);
-  k_emission_plan<<<1, 128, 0, c->stream>>>(c->d_inst, ninst, c->d_src, c->nsrc_total,
-                                            c->d_state, c->d_src_count, c->d_src_first,
-                                            c->d_buf_first, c->d_stats, nullptr, c->d_hist);
+  c->iteration = iteration;
+  k_begin_emission<<<1, kBeginThreads, 0, c->stream>>>(
+      c->d_inst, ninst, c->d_src, c->nsrc_total, c->d_state, c->d_src_count, c->d_src_first,
+      c->d_buf_first, c->d_stats, nullptr, c->d_hist, nullptr, 0u);
   CMI_CUDA(cudaGetLastError());
   uint32_t emitted = 0;
   CMI_CUDA(cudaMemcpyAsync(&emitted, &c->d_state->emit_total, sizeof(uint32_t),
@@ -1611,7 +1617,6 @@ int cmi_emit_photons(cmi_context *c, uint64_t seed, uint32_t iteration, cmi_phot
 
 int cmi_shoot_packets(cmi_context *c, uint64_t seed, uint32_t iteration, cmi_stats *stats) {
   CMI_TRY(check_ctx(c, false));
-  CMI_TRY(clear_flags(c));
   return run(c, 1, seed, iteration, false, stats);
 }
 
@@ -1658,7 +1663,7 @@ int cmi_transport_packets(cmi_context *c, int32_t instance, const cmi_photon *pa
   c->enqueued = 0;
   CMI_TRY(launch_plan(c, true));
   CMI_TRY(enqueue_rounds(c));
-  k_end_iteration<<<1, 128, 0, c->stream>>>(c->d_state, c->d_stats, ninst, 0);
+  k_end_iteration<<<1, 128, 0, c->stream>>>(c->d_state, c->d_stats, ninst, 0, nullptr);
   CMI_CUDA(cudaGetLastError());
   c->last_launches = c->enqueued + 3;
   CMI_TRY(ensure_host_stats(c, ninst));
@@ -1677,11 +1682,34 @@ int cmi_transport_packets(cmi_context *c, int32_t instance, const cmi_photon *pa
   return CMI_OK;
 }
 
-static int traverse(cmi_context *c, int32_t instance, uint32_t subgrid, int32_t input_direction,
-                    const cmi_photon *in, uint32_t n, cmi_photon *out_grouped,
-                    int32_t *out_dir_host, const uint8_t *enabled, uint32_t *out_count,
-                    uint32_t *num_done, int32_t max_steps, int32_t *cells, double *lengths,
-                    int32_t *num_steps) {
+// Results of a traversal, in front of its photons in the staging buffer; copied in as
+// zeros (with the enabled flags) and out with one copy each.
+struct TraverseHead {
+  uint32_t counts[28];
+  uint32_t done, err;
+  int32_t dir, steps;
+  uint8_t enabled[32];
+  uint32_t pad[8];
+};
+static_assert(sizeof(TraverseHead) == 192, "the photons behind it stay aligned");
+
+// pinned bytes for a call's copies: small ones pass through here (a pageable copy
+// waits on its own), larger ones go from and to the caller's memory
+constexpr size_t kPinnedMost = 1u << 20;
+
+static int ensure_pinned(cmi_context *c, size_t bytes) {
+  if (bytes <= c->h_pin_bytes) return CMI_OK;
+  if (c->h_pin) cudaFreeHost(c->h_pin);
+  c->h_pin = nullptr;
+  c->h_pin_bytes = 0;
+  const size_t grown = std::max<size_t>(bytes, 65536);
+  CMI_CUDA(cudaMallocHost((void **)&c->h_pin, grown));
+  c->h_pin_bytes = grown;
+  return CMI_OK;
+}
+
+static int check_traverse(cmi_context *c, int32_t instance, uint32_t subgrid,
+                          int32_t input_direction, const cmi_photon *in, uint32_t n) {
   CMI_TRY(check_ctx(c));
   CMI_TRY(check_instance(c, instance));
   const HostInstance &I = c->inst[instance];
@@ -1690,109 +1718,41 @@ static int traverse(cmi_context *c, int32_t instance, uint32_t subgrid, int32_t 
   if (input_direction < 0 || input_direction >= kNumDirections)
     return fail(CMI_ERR_INVALID_ARGUMENT, "input direction %d out of range", input_direction);
   if (n > 0 && !in) return fail(CMI_ERR_INVALID_ARGUMENT, "null input buffer");
-  CMI_TRY(clear_flags(c));
-  const size_t a16 = (sizeof(Packet64) * (size_t)n + 15) & ~(size_t)15;
-  const size_t bytes = 2 * a16 + 16 * (size_t)n + 27 * 4 + 256 + 16 * (size_t)std::max(max_steps, 0);
-  CMI_TRY(ensure_stage(c, bytes));
-  char *base = reinterpret_cast<char *>(c->d_stage);
-  Packet64 *d_in = reinterpret_cast<Packet64 *>(base);
-  Packet64 *d_out = reinterpret_cast<Packet64 *>(base + a16);
-  int32_t *d_dir = reinterpret_cast<int32_t *>(base + 2 * a16);
-  char *tail = base + 2 * a16 + (((size_t)n * 4 + 15) & ~(size_t)15);
-  uint32_t *d_counts = reinterpret_cast<uint32_t *>(tail);
-  uint32_t *d_done = d_counts + 28;
-  uint8_t *d_enabled = reinterpret_cast<uint8_t *>(d_counts + 32);
-  int32_t *d_steps = reinterpret_cast<int32_t *>(d_counts + 48);
-  int32_t *d_cells = reinterpret_cast<int32_t *>(d_counts + 64);
-  double *d_len = reinterpret_cast<double *>(
-      (reinterpret_cast<uintptr_t>(d_cells + std::max(max_steps, 1)) + 15) & ~(uintptr_t)15);
-  if (n > 0)
-    CMI_CUDA(cudaMemcpyAsync(d_in, in, sizeof(Packet64) * n, cudaMemcpyHostToDevice, c->stream));
-  if (enabled)
-    CMI_CUDA(cudaMemcpyAsync(d_enabled, enabled, 27, cudaMemcpyHostToDevice, c->stream));
-  TraverseParams t{};
+  return CMI_OK;
+}
+
+static int launch_traverse(cmi_context *c, TraverseParams &t, int32_t instance, uint32_t subgrid,
+                           int32_t input_direction) {
   t.subs = c->d_sub;
   t.inst = c->d_inst;
-  t.sub = I.first_sub + subgrid;
+  t.sub = c->inst[instance].first_sub + subgrid;
   t.input_direction = input_direction;
-  t.in = d_in;
-  t.n = n;
-  t.out = d_out;
-  t.out_dir = d_dir;
   t.kappa = c->d_kappa;
   t.nH = c->d_nH;
   t.xH = c->d_xH;
   t.J = c->d_J;
   t.max_padded = c->max_padded;
-  t.trace_cells = d_cells;
-  t.trace_len = d_len;
-  t.max_steps = max_steps;
-  t.trace_steps = num_steps ? d_steps : nullptr;
-  t.st = c->d_state;
   t.tables = c->tables;
-  const size_t smem = (c->fp32() ? 12 : 24) * (size_t)c->max_padded +
-                     (c->mixed() ? 8 * (size_t)c->max_faces : 0);
-  if (n > 0) {
-    const int grid = (int)((n + 255) / 256);
-    if (c->fp32()) {
-      CMI_CUDA(cudaFuncSetAttribute(k_traverse<kPk32>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      k_traverse<kPk32><<<grid, 256, smem, c->stream>>>(t);
-    } else if (c->mixed()) {
-      CMI_CUDA(cudaFuncSetAttribute(k_traverse<kPkM>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      k_traverse<kPkM><<<grid, 256, smem, c->stream>>>(t);
-    } else {
-      CMI_CUDA(cudaFuncSetAttribute(k_traverse<kPk64>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      k_traverse<kPk64><<<grid, 256, smem, c->stream>>>(t);
-    }
-    CMI_CUDA(cudaGetLastError());
+  // kappa and two FP32 tallies, or the FP64 fields and the face table
+  const size_t smem = (c->fp32() ? 12 : 16) * (size_t)c->max_padded +
+                      (c->mixed() ? 8 * (size_t)c->max_faces : 0);
+  const int grid = (int)((t.n + 255) / 256);
+  const void *fn = c->fp32()    ? (const void *)k_traverse<kPk32>
+                   : c->mixed() ? (const void *)k_traverse<kPkM>
+                                : (const void *)k_traverse<kPk64>;
+  if (!c->traverse_ready) {  // the largest any context may need: 8192 cells, 3 faces more
+    CMI_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 213 * 1024));
+    c->traverse_ready = true;
   }
-  if (out_grouped) {
-    k_partition<<<1, 256, 0, c->stream>>>(d_out, d_dir, n, enabled ? d_enabled : nullptr,
-                                          reinterpret_cast<Packet64 *>(d_in), d_counts, d_done);
-    CMI_CUDA(cudaGetLastError());
-  }
-  uint32_t flags = 0;
-  CMI_CUDA(cudaMemcpyAsync(&flags, &c->d_state->flags, sizeof(flags), cudaMemcpyDeviceToHost,
-                           c->stream));
-  uint32_t counts[28] = {0};
-  if (out_grouped) {
-    CMI_CUDA(cudaMemcpyAsync(counts, d_counts, sizeof(uint32_t) * 28, cudaMemcpyDeviceToHost,
-                             c->stream));
-  }
-  if (out_dir_host && n > 0)
-    CMI_CUDA(cudaMemcpyAsync(out_dir_host, d_dir, sizeof(int32_t) * n, cudaMemcpyDeviceToHost,
-                             c->stream));
-  int32_t steps = 0;
-  if (num_steps)
-    CMI_CUDA(cudaMemcpyAsync(&steps, d_steps, sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
-  CMI_CUDA(cudaStreamSynchronize(c->stream));
-  if (out_grouped) {
-    uint32_t kept = 0;
-    for (int d = 0; d < kNumDirections; ++d) {
-      out_count[d] = counts[d];
-      kept += counts[d];
-    }
-    uint32_t done = 0;
-    CMI_CUDA(cudaMemcpy(&done, d_done, sizeof(done), cudaMemcpyDeviceToHost));
-    if (num_done) *num_done = done;
-    if (kept > 0)
-      CMI_CUDA(cudaMemcpy(out_grouped, d_in, sizeof(Packet64) * kept, cudaMemcpyDeviceToHost));
-  } else if (n > 0 && out_dir_host) {
-    // single packet trace: photon comes back in place of the input
-    CMI_CUDA(cudaMemcpy(const_cast<cmi_photon *>(in), d_out, sizeof(Packet64) * n,
-                        cudaMemcpyDeviceToHost));
-  }
-  if (num_steps) {
-    *num_steps = steps;
-    const int32_t k = std::min(steps, max_steps);
-    if (k > 0) {
-      CMI_CUDA(cudaMemcpy(cells, d_cells, sizeof(int32_t) * k, cudaMemcpyDeviceToHost));
-      CMI_CUDA(cudaMemcpy(lengths, d_len, sizeof(double) * k, cudaMemcpyDeviceToHost));
-    }
-  }
+  if (c->fp32()) k_traverse<kPk32><<<grid, 256, smem, c->stream>>>(t);
+  else if (c->mixed()) k_traverse<kPkM><<<grid, 256, smem, c->stream>>>(t);
+  else k_traverse<kPk64><<<grid, 256, smem, c->stream>>>(t);
+  CMI_CUDA(cudaGetLastError());
+  return CMI_OK;
+}
+
+static int traverse_flags(uint32_t flags) {
+  if (flags & kFlagStageTimeout) return fail(CMI_ERR_DEVICE_TIMEOUT, "staging wait timed out");
   if (flags & kFlagWalkLimit) return fail(CMI_ERR_INVARIANT, "walk step bound exceeded");
   return CMI_OK;
 }
@@ -1802,8 +1762,56 @@ int cmi_traverse_buffer(cmi_context *c, int32_t instance, uint32_t subgrid,
                         const uint8_t *enabled, cmi_photon *out, uint32_t out_count[27],
                         uint32_t *num_done) {
   if (!out || !out_count) return fail(CMI_ERR_INVALID_ARGUMENT, "null output buffers");
-  return traverse(c, instance, subgrid, input_direction, in, n, out, nullptr, enabled,
-                  out_count, num_done, 0, nullptr, nullptr, nullptr);
+  CMI_TRY(check_traverse(c, instance, subgrid, input_direction, in, n));
+  // [head | photons, in and grouped | walked photons | directions]
+  const size_t pk = sizeof(Packet64) * (size_t)n, hd = sizeof(TraverseHead);
+  CMI_TRY(ensure_stage(c, hd + 2 * pk + 4 * (size_t)n + 64));
+  char *base = reinterpret_cast<char *>(c->d_stage);
+  TraverseHead *d_head = reinterpret_cast<TraverseHead *>(base);
+  Packet64 *d_in = reinterpret_cast<Packet64 *>(base + hd);
+  const bool small = hd + pk <= kPinnedMost;
+  CMI_TRY(ensure_pinned(c, hd + (small ? pk : 0)));
+  TraverseHead *h = reinterpret_cast<TraverseHead *>(c->h_pin);
+  std::memset(h, 0, hd);
+  for (int d = 0; d < kNumDirections; ++d) h->enabled[d] = enabled ? enabled[d] : 1;
+  if (small && n > 0) std::memcpy(c->h_pin + hd, in, pk);
+  CMI_CUDA(cudaMemcpyAsync(base, c->h_pin, hd + (small ? pk : 0), cudaMemcpyHostToDevice,
+                           c->stream));
+  if (!small) CMI_CUDA(cudaMemcpyAsync(d_in, in, pk, cudaMemcpyHostToDevice, c->stream));
+  if (n > 0) {
+    TraverseParams t{};
+    t.in = d_in;
+    t.n = n;
+    t.out = reinterpret_cast<Packet64 *>(base + hd + pk);
+    t.out_dir = reinterpret_cast<int32_t *>(base + hd + 2 * pk);
+    t.err = &d_head->err;
+    if (n <= 256u) {  // one block: it groups what it walked
+      t.grouped = d_in;
+      t.enabled = d_head->enabled;
+      t.counts = d_head->counts;
+      t.done = &d_head->done;
+    }
+    CMI_TRY(launch_traverse(c, t, instance, subgrid, input_direction));
+    if (n > 256u) {
+      k_partition<<<1, 256, 0, c->stream>>>(t.out, t.out_dir, n, d_head->enabled, d_in,
+                                            d_head->counts, &d_head->done);
+      CMI_CUDA(cudaGetLastError());
+    }
+  }
+  CMI_CUDA(cudaMemcpyAsync(c->h_pin, base, hd + (small ? pk : 0), cudaMemcpyDeviceToHost,
+                           c->stream));
+  CMI_CUDA(cudaStreamSynchronize(c->stream));
+  size_t kept = 0;
+  for (int d = 0; d < kNumDirections; ++d) {
+    out_count[d] = h->counts[d];
+    kept += h->counts[d];
+  }
+  if (num_done) *num_done = h->done;
+  if (kept > 0) {
+    if (small) std::memcpy(out, c->h_pin + hd, sizeof(Packet64) * kept);
+    else CMI_CUDA(cudaMemcpy(out, d_in, sizeof(Packet64) * kept, cudaMemcpyDeviceToHost));
+  }
+  return traverse_flags(h->err);
 }
 
 int cmi_trace_packet(cmi_context *c, int32_t instance, uint32_t subgrid, int32_t input_direction,
@@ -1813,8 +1821,39 @@ int cmi_trace_packet(cmi_context *c, int32_t instance, uint32_t subgrid, int32_t
     return fail(CMI_ERR_INVALID_ARGUMENT, "null photon or outputs");
   if (max_steps < 0 || (max_steps > 0 && (!cells || !lengths)))
     return fail(CMI_ERR_INVALID_ARGUMENT, "bad trace arrays");
-  return traverse(c, instance, subgrid, input_direction, photon, 1, nullptr, output_direction,
-                  nullptr, nullptr, nullptr, max_steps, cells, lengths, num_steps);
+  CMI_TRY(check_traverse(c, instance, subgrid, input_direction, photon, 1));
+  // [head | photon in | photon out | lengths | cells]
+  const size_t pk = sizeof(Packet64), hd = sizeof(TraverseHead);
+  CMI_TRY(ensure_stage(c, hd + 2 * pk + 12 * (size_t)std::max(max_steps, 1) + 64));
+  char *base = reinterpret_cast<char *>(c->d_stage);
+  TraverseHead *d_head = reinterpret_cast<TraverseHead *>(base);
+  TraverseParams t{};
+  t.in = reinterpret_cast<Packet64 *>(base + hd);
+  t.n = 1;
+  t.out = reinterpret_cast<Packet64 *>(base + hd + pk);
+  t.out_dir = &d_head->dir;
+  t.err = &d_head->err;
+  t.trace_len = reinterpret_cast<double *>(base + hd + 2 * pk);
+  t.trace_cells = reinterpret_cast<int32_t *>(t.trace_len + std::max(max_steps, 1));
+  t.max_steps = max_steps;
+  t.trace_steps = &d_head->steps;
+  CMI_TRY(ensure_pinned(c, hd + 2 * pk));
+  TraverseHead *h = reinterpret_cast<TraverseHead *>(c->h_pin);
+  std::memset(h, 0, hd);
+  std::memcpy(c->h_pin + hd, photon, pk);
+  CMI_CUDA(cudaMemcpyAsync(base, c->h_pin, hd + pk, cudaMemcpyHostToDevice, c->stream));
+  CMI_TRY(launch_traverse(c, t, instance, subgrid, input_direction));
+  CMI_CUDA(cudaMemcpyAsync(c->h_pin, base, hd + 2 * pk, cudaMemcpyDeviceToHost, c->stream));
+  CMI_CUDA(cudaStreamSynchronize(c->stream));
+  std::memcpy(photon, c->h_pin + hd + pk, pk);
+  *output_direction = h->dir;
+  *num_steps = h->steps;
+  const int32_t k = std::min(h->steps, max_steps);
+  if (k > 0) {
+    CMI_CUDA(cudaMemcpy(cells, t.trace_cells, sizeof(int32_t) * k, cudaMemcpyDeviceToHost));
+    CMI_CUDA(cudaMemcpy(lengths, t.trace_len, sizeof(double) * k, cudaMemcpyDeviceToHost));
+  }
+  return traverse_flags(h->err);
 }
 
 int cmi_compute_neutral_fraction_subgrids(cmi_context *c, int32_t instance,

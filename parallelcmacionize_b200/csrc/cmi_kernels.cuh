@@ -126,7 +126,22 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t *w
 // ---------------------------------------------------------------------------
 // iteration bookkeeping
 // ---------------------------------------------------------------------------
-__global__ void k_begin_iteration(RoundState *st, DevStats *stats, int ninst) {
+// One of the kPathShares shares that the path kernel cuts N packets into.
+constexpr int kPathThreads = 128;
+constexpr int kPathWarps = kPathThreads / 32;
+struct PathShare {
+  uint32_t begin, size;
+  __device__ __forceinline__ PathShare(uint32_t n, uint32_t k) {
+    const uint64_t part = ((uint64_t)n / kPathShares + 31u) & ~31ull;
+    const uint64_t b = min((uint64_t)n, k * part);
+    const uint64_t e = k + 1u == kPathShares ? (uint64_t)n : min((uint64_t)n, b + part);
+    begin = (uint32_t)b;
+    size = (uint32_t)(e - b);
+  }
+};
+
+// Counters of an iteration back to zero.
+__device__ __forceinline__ void reset_iteration(RoundState *st, DevStats *stats, int ninst) {
   for (int i = threadIdx.x; i < ninst; i += blockDim.x) {
     DevStats z = {};
     stats[i] = z;
@@ -139,20 +154,45 @@ __global__ void k_begin_iteration(RoundState *st, DevStats *stats, int ninst) {
     st->chunk_next = 0;
     st->total_in = 0;
   }
-  if (threadIdx.x < kPathShares) st->share_next[threadIdx.x] = 0;
 }
 
-__global__ void k_end_iteration(RoundState *st, DevStats *stats, int ninst, int advance) {
-  const uint32_t leftover = st->total_in ? kFlagLeftover : 0u;
+__global__ void k_begin_iteration(RoundState *st, DevStats *stats, int ninst) {
+  reset_iteration(st, stats, ninst);
+}
+
+// Flags and rounds into the statistics, and those into the caller's pinned array
+// (host, may be null; a copy of its own would cost a launch and a copy engine's turn).
+// One block.
+__device__ __forceinline__ void finish_iteration(RoundState *st, DevStats *stats, int ninst,
+                                                 bool advance, DevStats *host) {
+  const uint32_t leftover = __ldcg(&st->total_in) ? kFlagLeftover : 0u;
+  const uint32_t flags = __ldcg(&st->flags) | leftover;
+  const uint32_t rounds = __ldcg(&st->rounds_active), slot = __ldcg(&st->slot);
+  static_assert(sizeof(DevStats) == 64, "copied as four vectors");
   for (int i = threadIdx.x; i < ninst; i += blockDim.x) {
-    stats[i].flags |= st->flags | leftover;
-    stats[i].rounds = st->rounds_active;
+    DevStats s;
+    uint4 *v = reinterpret_cast<uint4 *>(&s);
+    for (int k = 0; k < 4; ++k) v[k] = __ldcg(reinterpret_cast<const uint4 *>(stats + i) + k);
+    s.flags |= flags;
+    s.rounds = rounds;
+    for (int k = 0; k < 4; ++k) {
+      reinterpret_cast<uint4 *>(stats + i)[k] = v[k];
+      if (host) reinterpret_cast<uint4 *>(host + (size_t)slot * ninst + i)[k] = v[k];
+    }
   }
   __syncthreads();
   if (threadIdx.x == 0) {
-    st->flags |= leftover;
-    if (advance) st->iteration += 1;
+    st->flags = flags;
+    if (advance) {
+      st->iteration += 1;
+      st->slot = slot + 1;
+    }
   }
+}
+
+__global__ void k_end_iteration(RoundState *st, DevStats *stats, int ninst, int advance,
+                                DevStats *host) {
+  finish_iteration(st, stats, ninst, advance != 0, host);
 }
 
 // Condition of the graph's round loop: another walk when the last plan left
@@ -174,10 +214,38 @@ __global__ void k_round_gate(RoundState *st, cudaGraphConditionalHandle h, uint3
 // the bucket histogram of its subgrid and records where in that bucket the
 // source's packets start, so the emitted packets can be written in sorted
 // order (k_emit_philox_direct) without appends or a scatter.
-__global__ void k_emission_plan(const DevInstance *inst, int ninst, const DevSource *src,
-                                int nsrc_total, RoundState *st, uint64_t *src_count,
-                                uint64_t *src_first, uint64_t *buf_first, DevStats *stats,
-                                uint32_t *src_rank0, uint32_t *hist) {
+// It begins the iteration: counters, and the seed and iteration of a new call (args,
+// may be null: set by the caller's copies).  path_ctas: CTAs of the path kernel, whose
+// warps hold a first claim of 32 packets each without asking.
+constexpr int kBeginThreads = 256;
+__device__ __forceinline__ uint64_t warp_scan64(uint64_t v) {  // inclusive
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint64_t y = __shfl_up_sync(kFull, v, o);
+    if ((threadIdx.x & 31) >= o) v += y;
+  }
+  return v;
+}
+
+__global__ void __launch_bounds__(kBeginThreads)
+    k_begin_emission(const DevInstance *inst, int ninst, const DevSource *src, int nsrc_total,
+                     RoundState *st, uint64_t *src_count, uint64_t *src_first,
+                     uint64_t *buf_first, DevStats *stats, uint32_t *src_rank0, uint32_t *hist,
+                     const RunArgs *args, uint32_t path_ctas) {
+  __shared__ uint64_t part[2][kBeginThreads / 32];
+  reset_iteration(st, stats, ninst);
+  if (args && threadIdx.x == 0) {
+    const volatile RunArgs *a = args;
+    const uint32_t ticket = a->ticket;
+    if (ticket != st->ticket) {
+      st->seed = a->seed;
+      st->iteration = a->iteration;
+      st->flags = 0;
+      st->slot = 0;
+      st->ticket = ticket;
+    }
+  }
+  __syncthreads();
   const uint64_t seed = st->seed;
   const uint32_t it = st->iteration;
   for (int i = threadIdx.x; i < ninst; i += blockDim.x) {
@@ -217,18 +285,45 @@ __global__ void k_emission_plan(const DevInstance *inst, int ninst, const DevSou
     stats[i].emitted = I.num_photon;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    uint64_t acc = 0, bacc = 0;
-    for (int s = 0; s < nsrc_total; ++s) {
-      src_first[s] = acc;
-      buf_first[s] = bacc;
-      acc += src_count[s];
-      bacc += (src_count[s] + 199) / 200;
+  // first packet and first 200-packet buffer of every source
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint64_t acc = 0, bacc = 0;
+  for (int s0 = 0; s0 < nsrc_total; s0 += kBeginThreads) {
+    const int s = s0 + (int)threadIdx.x;
+    const uint64_t n = s < nsrc_total ? src_count[s] : 0u, nb = (n + 199) / 200;
+    const uint64_t x = warp_scan64(n), xb = warp_scan64(nb);
+    if (lane == 31) {
+      part[0][warp] = x;
+      part[1][warp] = xb;
     }
+    __syncthreads();
+    uint64_t before = 0, bbefore = 0, all = 0, ball = 0;
+    for (int w = 0; w < kBeginThreads / 32; ++w) {
+      if (w < warp) {
+        before += part[0][w];
+        bbefore += part[1][w];
+      }
+      all += part[0][w];
+      ball += part[1][w];
+    }
+    if (s < nsrc_total) {
+      src_first[s] = acc + before + x - n;
+      buf_first[s] = bacc + bbefore + xb - nb;
+    }
+    acc += all;
+    bacc += ball;
+    __syncthreads();
+  }
+  if (threadIdx.x < kPathShares) {
+    const uint32_t k = threadIdx.x;
+    const uint32_t ctas = path_ctas > k ? (path_ctas - k + kPathShares - 1) / kPathShares : 0u;
+    const PathShare share((uint32_t)acc, k);
+    st->share_next[k] = min(share.size, ctas * kPathWarps * 32u);
+  }
+  if (threadIdx.x == 0) {
     src_first[nsrc_total] = acc;
     buf_first[nsrc_total] = bacc;
     st->emit_total = (uint32_t)acc;
-    st->arena_count = 0;
     if (src_rank0) {  // sources in order: ranks inside each subgrid's bucket
       for (int s = 0; s < nsrc_total; ++s) {
         const uint32_t sub = src[s].subgrid;
@@ -1563,6 +1658,10 @@ struct BalanceParams {
   const uint32_t *hot;
   uint32_t copies;
   bool fixed;
+  // the last block ends the iteration (st may be null)
+  RoundState *st;
+  int ninst;
+  DevStats *host;
 };
 
 template <int kForm>
@@ -1571,12 +1670,13 @@ __global__ void __launch_bounds__(256) k_balance(BalanceParams prm) {
   const uint32_t s = prm.first_sub + blockIdx.x;
   const DevSubgrid &S = prm.subs[s];
   const DevInstance &I = prm.inst[S.instance];
-  if (I.frozen) return;  // converged: x_H kept, J is zero (no packets)
+  // converged: x_H kept, J is zero (no packets)
+  const int ncells = I.frozen ? 0 : S.ncells;
   const double jfac = (prm.jfac_override >= 0.) ? prm.jfac_override : I.jfac;
   const double alpha = I.alpha;
   const double sigma = I.sigma;
   double dx = 0.;
-  const int end = min(S.ncells, (int)(blockIdx.y + 1) * kBalanceCells);
+  const int end = min(ncells, (int)(blockIdx.y + 1) * kBalanceCells);
   for (int c = (int)blockIdx.y * kBalanceCells + threadIdx.x; c < end; c += blockDim.x) {
     const int64_t i = S.field_offset + c;
     double J = prm.J[i];
@@ -1610,8 +1710,19 @@ __global__ void __launch_bounds__(256) k_balance(BalanceParams prm) {
   if (threadIdx.x == 0) {
     double t = 0.;
     for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += red[w];
-    if (prm.stats) atomicAdd(&prm.stats[S.instance].dx_sum, t);
+    if (prm.stats && t != 0.) atomicAdd(&prm.stats[S.instance].dx_sum, t);
   }
+  if (!prm.st) return;
+  __shared__ bool last;
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(&prm.st->blocks_done, 1u) + 1u == gridDim.x * gridDim.y;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  finish_iteration(prm.st, prm.stats, prm.ninst, true, prm.host);
+  if (threadIdx.x == 0) prm.st->blocks_done = 0u;
 }
 
 // ---------------------------------------------------------------------------
@@ -1692,10 +1803,54 @@ struct TraverseParams {
   double *trace_len;
   int32_t max_steps;
   int32_t *trace_steps;
-  RoundState *st;
+  uint32_t *err;          // CMI_FLAG_* bits
+  // grouping by output direction in the same launch (one block; may be null)
+  Packet64 *grouped;
+  const uint8_t *enabled;
+  uint32_t *counts, *done;
   DirectionTables tables;
 };
 
+// Where the photons of a block go: stable grouping by direction of up to kThreads
+// photons, one per thread (d < 0: none).  Returns the thread's place, kNone for a
+// disabled group; counts and done as do_photon_traversal's buffers.
+template <int kThreads>
+__device__ __forceinline__ uint32_t group_place(int d, const uint8_t *enabled, uint32_t *counts,
+                                                uint32_t *done) {
+  __shared__ uint32_t cnt[kThreads / 32][32], base[32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  cnt[warp][lane] = 0u;
+  __syncwarp();
+  const unsigned peers = __match_any_sync(kFull, d);
+  const uint32_t rank = (uint32_t)__popc(peers & ((1u << lane) - 1u));
+  if (d >= 0 && rank == 0u) cnt[warp][d] = (uint32_t)__popc(peers);
+  __syncthreads();
+  if (warp == 0) {  // lane: direction
+    uint32_t acc = 0;
+    for (int w = 0; w < kThreads / 32; ++w) {
+      const uint32_t c = cnt[w][lane];
+      cnt[w][lane] = acc;
+      acc += c;
+    }
+    const bool on = lane < kNumDirections && (enabled == nullptr || enabled[lane] != 0);
+    uint32_t x = on ? acc : 0u;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(kFull, x, o);
+      if (lane >= o) x += y;
+    }
+    base[lane] = on ? x - acc : kNone;
+    const uint32_t dropped = __reduce_add_sync(kFull, on ? 0u : acc);
+    if (lane < kNumDirections) counts[lane] = on ? acc : 0u;
+    if (lane == 0) *done = dropped;
+  }
+  __syncthreads();
+  return d >= 0 && base[d] != kNone ? base[d] + cnt[warp][d] + rank : kNone;
+}
+
+// One launch walks and groups a buffer of up to 256 photons (the reference's holds 200);
+// bound by latency: with the fields by bulk copy, no tally of its own and the copies of
+// a call joined, 200 photons through 16^3 cells take 38 us a call, 91 before (B200).
 // K: the transport's packet record.  The mixed-precision walk takes each
 // photon's own cross section: its cell opacity is (float)(sigma n x) of the
 // photon's sigma (the production kappa when sigma is the instance's), and it
@@ -1710,27 +1865,34 @@ __global__ void __launch_bounds__(256) k_traverse(TraverseParams prm) {
   float *s_kappa = reinterpret_cast<float *>(smem_raw);
   float *s_hi = s_kappa + P;
   float *s_lo = s_hi + P;
+  // FP64 fields, by bulk copy; path lengths go straight to J: a buffer's photons touch
+  // a part of the cells, once or twice each, so a tally of its own would be zeroed and
+  // flushed mostly for nothing
   double *s_n = reinterpret_cast<double *>(smem_raw);
   double *s_x = s_n + P;
-  double *s_J = s_x + P;
-  double *s_faces = s_J + P;  // mixed walk: face table (nx + ny + nz + 3 entries)
+  double *s_faces = s_x + P;  // mixed walk: face table (nx + ny + nz + 3 entries)
+  __shared__ alignas(8) unsigned long long mbar;
+  double *J = prm.J + S.field_offset;
   if (threadIdx.x < sizeof(DirectionTables) / 4) {
     reinterpret_cast<uint32_t *>(&tab)[threadIdx.x] =
         reinterpret_cast<const uint32_t *>(&prm.tables)[threadIdx.x];
   }
-  for (int c = threadIdx.x; c < S.ncells; c += blockDim.x) {
-    if (kF32) {
+  if (kF32) {
+    for (int c = threadIdx.x; c < S.ncells; c += blockDim.x) {
       s_kappa[c] = prm.kappa[S.field_offset + c];
       s_hi[c] = 0.f;
       s_lo[c] = 0.f;
-    } else {
-      s_n[c] = prm.nH[S.field_offset + c];
-      s_x[c] = prm.xH[S.field_offset + c];
-      s_J[c] = 0.;
     }
+  } else if (threadIdx.x == 0) {
+    mbar_init(&mbar, 1);
+    const uint32_t bytes = (uint32_t)S.padded_cells * 8u;
+    mbar_expect_tx(&mbar, 2u * bytes);
+    tma_load_1d(s_n, prm.nH + S.field_offset, bytes, &mbar);
+    tma_load_1d(s_x, prm.xH + S.field_offset, bytes, &mbar);
   }
   if (K == kPkM) fill_faces(s_faces, S.ncell, S.cell_size, threadIdx.x, blockDim.x);
   __syncthreads();
+  if (!kF32) mbar_wait_bounded(&mbar, 0u, prm.err);
   View32 v32;
   View64 v64;
   for (int a = 0; a < 3; ++a) {
@@ -1751,15 +1913,16 @@ __global__ void __launch_bounds__(256) k_traverse(TraverseParams prm) {
   tally32.scale = 1.f;
   v64.nH = s_n;
   v64.xH = s_x;
-  v64.J = s_J;
+  v64.J = J;
   const int limit = S.ncell[0] + S.ncell[1] + S.ncell[2] + 3;
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  Packet64 ph{};
+  int result = kInside;
   if (i < prm.n) {
-    Packet64 ph = prm.in[i];
+    ph = prm.in[i];
     ph.meta = (uint32_t)prm.input_direction;
     const bool tracing = (i == 0 && prm.trace_steps != nullptr);
     int status, nsteps = 0;
-    int result = kInside;
     if (kF32) {
       Packet32 pk;
       for (int a = 0; a < 3; ++a) {
@@ -1814,7 +1977,7 @@ __global__ void __launch_bounds__(256) k_traverse(TraverseParams prm) {
         float lf;
         double len;
         status = w.step_k(vm, k, cell, lf, &len);
-        atomicAdd(&s_J[cell], len * sg * wt);
+        atomicAdd(&J[cell], len * sg * wt);
         if (tracing && nsteps < prm.max_steps) {
           prm.trace_cells[nsteps] = cell;
           prm.trace_len[nsteps] = len;
@@ -1844,22 +2007,27 @@ __global__ void __launch_bounds__(256) k_traverse(TraverseParams prm) {
       if (status == kExited) result = tab.mask_dir[w.exit_mask(v64)];
     }
     if (status == kDrop || result >= kNumDirections) {
-      atomicOr(&prm.st->flags, kFlagWalkLimit);
+      atomicOr(prm.err, kFlagWalkLimit);
       result = kInside;
     }
     ph.meta = 0u;
-    prm.out[i] = ph;
-    prm.out_dir[i] = result;
+    if (!prm.grouped) {
+      store_packet(prm.out + i, ph);
+      prm.out_dir[i] = result;
+    }
     if (tracing) *prm.trace_steps = nsteps;
   }
-  __syncthreads();
-  const double sw = prm.inst[S.instance].sigma;
-  for (int c = threadIdx.x; c < S.ncells; c += blockDim.x) {
-    if (kF32) {
+  if (prm.grouped) {
+    const uint32_t place = group_place<256>(i < prm.n ? result : -1, prm.enabled, prm.counts,
+                                            prm.done);
+    if (place != kNone) store_packet(prm.grouped + place, ph);
+  }
+  if (kF32) {
+    __syncthreads();
+    const double sw = prm.inst[S.instance].sigma;
+    for (int c = threadIdx.x; c < S.ncells; c += blockDim.x) {
       const double v = ((double)s_hi[c] + (double)s_lo[c]) * sw;
-      if (v != 0.) atomicAdd(&prm.J[S.field_offset + c], v);
-    } else {
-      if (s_J[c] != 0.) atomicAdd(&prm.J[S.field_offset + c], s_J[c]);
+      if (v != 0.) atomicAdd(&J[c], v);
     }
   }
 }
@@ -1877,15 +2045,22 @@ __global__ void __launch_bounds__(256) k_partition(const Packet64 *photons,
   for (int d = 0; d < kNumDirections; ++d) cnt[threadIdx.x][d] = 0;
   for (uint32_t i = b; i < e; ++i) cnt[threadIdx.x][dirs[i]] += 1;
   __syncthreads();
-  if (threadIdx.x < kNumDirections) {
-    const int d = threadIdx.x;
+  // exclusive prefix over the threads, a warp per direction
+  const int lane = threadIdx.x & 31;
+  for (int d = threadIdx.x >> 5; d < kNumDirections; d += 8) {
     uint32_t acc = 0;
-    for (int t = 0; t < 256; ++t) {
+    for (int t = lane; t < 256; t += 32) {
       const uint32_t c = cnt[t][d];
-      cnt[t][d] = acc;
-      acc += c;
+      uint32_t x = c;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(kFull, x, o);
+        if (lane >= o) x += y;
+      }
+      cnt[t][d] = acc + x - c;
+      acc += __shfl_sync(kFull, x, 31);
     }
-    base[d] = acc;  // total of direction d for now
+    if (lane == 0) base[d] = acc;  // total of direction d for now
   }
   __syncthreads();
   if (threadIdx.x == 0) {

@@ -27,7 +27,7 @@
 //
 // Bound by instruction issue and lane divergence (log-normal 128^3, mixed: 54% of
 // issue slots, 19 of 32 lanes, L1 58% and L2 37% of peak).  Against the wavefront, us
-// per iteration: 32^3, 2e4 packets 212 -> 62; stromgren 64^3, 1e6 907 -> 335;
+// per iteration: 32^3, 2e4 packets 216 -> 60; stromgren 64^3, 1e6 907 -> 335;
 // log-normal 128^3, 1e7 4060 -> 2034; 256^3, 1e8 53000 -> 32400; 12 uneven instances
 // 6860 -> 4050; FP64 walk, 64^3, 1e6 1276 -> 242.
 #pragma once
@@ -74,8 +74,6 @@ struct PathParams {
   uint32_t round_cap;             // most subgrid visits of one packet
 };
 
-constexpr int kPathThreads = 128;
-constexpr int kPathWarps = kPathThreads / 32;
 constexpr int kPathFree = 4;      // lane status beyond WalkStatus and kDrop
 constexpr int kPathStretch = 64;  // steps between two looks at the step bound
 // A warp turns to its lanes at subgrid faces once this many more lanes wait than it
@@ -105,7 +103,7 @@ struct PathShared {
   uint32_t again[32];      // reemissions in this subgrid
   // the warp's work: claimed packets, end of the current source's, queue
   uint64_t inst_first;     // first packet of the current instance
-  uint32_t inst, share, job, job_end, src_begin, src_end, q_at, q_n, exhausted;
+  uint32_t inst, fresh, share, job, job_end, src_begin, src_end, q_at, q_n, exhausted;
   // per lane: packets absorbed, escaped and re-emitted, most subgrids entered
   uint32_t absorbed[32], escaped[32], reemitted[32], most[32];
 };
@@ -783,14 +781,21 @@ __device__ __noinline__ void path_emit(const PathParams &prm, PathShared &sh, do
     // Guided claims, about half an even part of what is left of the share, then of the
     // next share with anything left.  CTAs start on different shares, so that they
     // spread over the sources: the cells around one take every packet it emits.
-    const uint32_t part = (uint32_t)(((uint64_t)N / kPathShares + 31u) & ~31ull);
     uint32_t j0 = 0, j1 = 0, own = sh.share;
-    for (;;) {
+    if (sh.fresh) {
+      // the first claim is the warp's by its place (k_begin_emission counts it)
+      const PathShare mine(N, own);
+      const uint32_t q = (blockIdx.x / kPathShares * kPathWarps + (threadIdx.x >> 5)) * 32u;
+      j0 = mine.begin + min(q, mine.size);
+      j1 = mine.begin + min(q + 32u, mine.size);
+      __syncwarp();
+      if (lane == 0) sh.fresh = 0u;
+    }
+    while (j0 >= j1) {
       // what is left of share (own + lane), seen by lane
       const uint32_t k = (own + (uint32_t)lane) % kPathShares;
-      const uint64_t b = min((uint64_t)N, (uint64_t)k * part);
-      const uint64_t e = k + 1u == kPathShares ? (uint64_t)N : min((uint64_t)N, b + part);
-      const uint32_t size = (uint32_t)(e - b);
+      const PathShare there(N, k);
+      const uint32_t size = there.size;
       const uint32_t taken =
           lane < kPathShares ? *(volatile uint32_t *)&st->share_next[k] : size;
       const unsigned open = __ballot_sync(kFull, taken < size);
@@ -800,13 +805,12 @@ __device__ __noinline__ void path_emit(const PathParams &prm, PathShared &sh, do
         const uint32_t jn = min(256u, max(32u, ((size - taken) * (uint32_t)kPathShares /
                                                 (2u * gridDim.x * kPathWarps)) & ~31u));
         const uint32_t q = atomicAdd(&st->share_next[k], jn);
-        j0 = (uint32_t)b + min(q, size);
-        j1 = (uint32_t)b + min(q + jn, size);
+        j0 = there.begin + min(q, size);
+        j1 = there.begin + min(q + jn, size);
       }
       j0 = __shfl_sync(kFull, j0, first);
       j1 = __shfl_sync(kFull, j1, first);
       own = (own + (uint32_t)first) % kPathShares;
-      if (j0 < j1) break;
     }
     if (lane == 0) sh.share = own;
     if (j0 >= j1) {
@@ -883,6 +887,7 @@ __global__ void __launch_bounds__(kPathThreads, kMinBlocks) k_path(const __grid_
   const uint32_t copy = (blockIdx.x * kPathWarps + (uint32_t)warp) % prm.copies;
   if (lane == 0) {
     sh.inst = kNone;
+    sh.fresh = 1u;
     sh.share = blockIdx.x % (uint32_t)kPathShares;
     sh.job = sh.job_end = sh.src_begin = sh.src_end = sh.q_at = sh.q_n = sh.exhausted = 0u;
   }
