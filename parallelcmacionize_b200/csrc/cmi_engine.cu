@@ -514,10 +514,14 @@ int upload_tables(cmi_context *c) {
   return CMI_OK;
 }
 
+dim3 field_grid(const HostInstance &I) {
+  return dim3(I.nsub, (unsigned)((I.padded_per_sub + kFieldCells - 1) / kFieldCells));
+}
+
 int refresh_kappa(cmi_context *c, int32_t i, cudaStream_t s = nullptr) {
   if (!c->uses_kappa()) return CMI_OK;
   const HostInstance &I = c->inst[i];
-  k_kappa<<<I.nsub, 256, 0, s ? s : c->stream>>>(c->d_sub, c->d_inst, I.first_sub, c->d_nH,
+  k_kappa<<<field_grid(I), 256, 0, s ? s : c->stream>>>(c->d_sub, c->d_inst, I.first_sub, c->d_nH,
                                                  c->d_xH, c->d_kappa);
   CMI_CUDA(cudaGetLastError());
   return CMI_OK;
@@ -1360,7 +1364,7 @@ static int copy_field_in(cmi_context *c, int32_t instance, int32_t layout, int32
     lp.ncell[a] = I.desc.ncell[a];
   }
   lp.layout = layout;
-  k_fields_in<<<I.nsub, 256, 0, s>>>(lp, dsrc, dst);
+  k_fields_in<<<field_grid(I), 256, 0, s>>>(lp, dsrc, dst);
   CMI_CUDA(cudaGetLastError());
   return CMI_OK;
 }
@@ -1377,7 +1381,7 @@ static int copy_field_out(cmi_context *c, int32_t instance, int32_t layout, int3
     lp.ncell[a] = I.desc.ncell[a];
   }
   lp.layout = layout;
-  k_fields_out<<<I.nsub, 256, 0, c->stream>>>(lp, src, ddst);
+  k_fields_out<<<field_grid(I), 256, 0, c->stream>>>(lp, src, ddst);
   CMI_CUDA(cudaGetLastError());
   if (memory == CMI_MEMORY_HOST) {
     CMI_CUDA(cudaMemcpyAsync(dst, c->d_stage, sizeof(double) * I.ncells, cudaMemcpyDeviceToHost,

@@ -1751,10 +1751,15 @@ struct LayoutParams {
   int layout;
 };
 
+// Grid: subgrids x blocks of kFieldCells cells of one (one block per subgrid left most
+// SMs idle on few large subgrids: 4^3 of 16^3 cells took 14 us, 6 now).
+constexpr int kFieldCells = 1024;
+
 __global__ void k_fields_in(LayoutParams lp, const double *src, double *dst) {
   const uint32_t ls = blockIdx.x;
   const DevSubgrid &S = lp.subs[lp.first_sub + ls];
-  for (int c = threadIdx.x; c < S.ncells; c += blockDim.x) {
+  const int end = min(S.ncells, (int)(blockIdx.y + 1) * kFieldCells);
+  for (int c = (int)blockIdx.y * kFieldCells + threadIdx.x; c < end; c += blockDim.x) {
     dst[S.field_offset + c] = src[layout_index(S, ls, c, lp.layout, lp.ns, lp.ncell)];
   }
 }
@@ -1762,7 +1767,8 @@ __global__ void k_fields_in(LayoutParams lp, const double *src, double *dst) {
 __global__ void k_fields_out(LayoutParams lp, const double *src, double *dst) {
   const uint32_t ls = blockIdx.x;
   const DevSubgrid &S = lp.subs[lp.first_sub + ls];
-  for (int c = threadIdx.x; c < S.ncells; c += blockDim.x) {
+  const int end = min(S.ncells, (int)(blockIdx.y + 1) * kFieldCells);
+  for (int c = (int)blockIdx.y * kFieldCells + threadIdx.x; c < end; c += blockDim.x) {
     dst[layout_index(S, ls, c, lp.layout, lp.ns, lp.ncell)] = src[S.field_offset + c];
   }
 }
@@ -1771,7 +1777,8 @@ __global__ void k_kappa(const DevSubgrid *subs, const DevInstance *inst, uint32_
                         const double *nH, const double *xH, float *kappa) {
   const DevSubgrid &S = subs[first_sub + blockIdx.x];
   const double sigma = inst[S.instance].sigma;
-  for (int c = threadIdx.x; c < S.padded_cells; c += blockDim.x) {
+  const int end = min(S.padded_cells, (int)(blockIdx.y + 1) * kFieldCells);
+  for (int c = (int)blockIdx.y * kFieldCells + threadIdx.x; c < end; c += blockDim.x) {
     const int64_t i = S.field_offset + c;
     kappa[i] = (c < S.ncells) ? (float)(sigma * nH[i] * xH[i]) : 0.f;
   }

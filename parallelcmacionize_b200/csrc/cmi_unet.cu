@@ -1733,6 +1733,61 @@ __global__ void k_nrel(const double *nH, float *nrel, long long n, double inv_nr
     nrel[i] = (float)__dmul_rn(nH[i], inv_nref);
 }
 
+// The midpoint sum along one ray, sample k at t = (k + 1/2) inv.  Bound by instruction
+// issue (64^3, 4 sources: 9e7 samples; 33 instructions each and 139 us with clamps and a
+// predicated tail, 165 us with conversions and single loads, 124 us like this), so a
+// sample is kept short:
+//  * no conversions (a quarter of the rate): t counts in FP32, exactly, and adding
+//    1.5 2^23 rounding down leaves the floor of a coordinate in the mantissa;
+//  * kClamp: only for sources at or outside a face of the box; clamping to [0, n - 1/2]
+//    before the floor gives the cell that clamping the floor to [0, n - 1] gives.
+// The loads of eight samples are on the way together; the sum keeps its order.
+template <bool kClamp>
+__device__ __forceinline__ float march_sample(const FeatureArgs &a, const float sf[3],
+                                              const float dc[3], float t) {
+  int c3[3];
+#pragma unroll
+  for (int m = 0; m < 3; ++m) {
+    float x = __fadd_rn(sf[m], __fmul_rn(t, dc[m]));
+    if (kClamp) x = fminf(fmaxf(x, 0.f), (float)a.n3[m] - 0.5f);
+    c3[m] = __float_as_int(__fadd_rd(x, 12582912.f));
+  }
+  constexpr unsigned kBias = 0x4B400000u;  // of each c3, taken off the sum at once
+  const unsigned n1 = (unsigned)a.n3[1], n2 = (unsigned)a.n3[2];
+  const unsigned off = (kBias * n1 + kBias) * n2 + kBias;
+  return __ldg(a.nrel + (((unsigned)c3[0] * n1 + (unsigned)c3[1]) * n2 + (unsigned)c3[2] - off));
+}
+template <bool kClamp>
+__device__ __forceinline__ float march(const FeatureArgs &a, const float sf[3], const float dc[3],
+                                       float rh, float inv, int nstep) {
+  constexpr int kBatch = 8;
+  float col = 0.f, kf = 0.5f;
+  auto add = [&](float n, float t) {
+    const float rr = __fmul_rn(t, rh);
+    col = __fadd_rn(col, __fmul_rn(__fmul_rn(n, n), __fmul_rn(rr, rr)));
+  };
+  int k = 0;
+#pragma unroll 1
+  for (; k + kBatch <= nstep; k += kBatch) {
+    float n[kBatch], t[kBatch];
+#pragma unroll
+    for (int j = 0; j < kBatch; ++j) {
+      t[j] = __fmul_rn(__fadd_rn(kf, (float)j), inv);
+      n[j] = march_sample<kClamp>(a, sf, dc, t[j]);
+    }
+    kf = __fadd_rn(kf, (float)kBatch);
+#pragma unroll
+    for (int j = 0; j < kBatch; ++j) add(n[j], t[j]);
+  }
+#pragma unroll 1
+  for (; k < nstep; ++k) {
+    const float t = __fmul_rn(kf, inv);
+    kf = __fadd_rn(kf, 1.f);
+    add(march_sample<kClamp>(a, sf, dc, t), t);
+  }
+  return col;
+}
+
 __global__ void k_features(FeatureArgs a) {
   const long long nvox = (long long)a.dims[0] * a.dims[1] * a.dims[2];
   const double hmin = fmin(a.cell[0], fmin(a.cell[1], a.cell[2]));
@@ -1741,8 +1796,9 @@ __global__ void k_features(FeatureArgs a) {
   const float hstep = 0.5f;
   for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < nvox;
        v += (long long)gridDim.x * blockDim.x) {
-    const int i3[3] = {(int)(v / ((long long)a.dims[0] * a.dims[1])),
-                       (int)((v / a.dims[0]) % a.dims[1]), (int)(v % a.dims[0])};
+    const unsigned row = (unsigned)v / (unsigned)a.dims[0];  // at most 2^31 cells
+    const int i3[3] = {(int)(row / (unsigned)a.dims[1]), (int)(row % (unsigned)a.dims[1]),
+                       (int)((unsigned)v % (unsigned)a.dims[0])};
     double flux = 0., strom = 0.;
     for (int s = 0; s < a.nsrc; ++s) {
       const double *S = a.src + 4 * s;
@@ -1764,18 +1820,11 @@ __global__ void k_features(FeatureArgs a) {
       const int nstep = max(1, (int)ceilf(__fdiv_rn(rh, hstep)));
       const float inv = __frcp_rn((float)nstep);
       const float sf[3] = {(float)sc[0], (float)sc[1], (float)sc[2]};
-      float col = 0.f;
-      for (int k = 0; k < nstep; ++k) {
-        const float t = __fmul_rn(__fadd_rn((float)k, 0.5f), inv);
-        int c3[3];
-        for (int m = 0; m < 3; ++m) {
-          const int ci = (int)floorf(__fadd_rn(sf[m], __fmul_rn(t, dc[m])));
-          c3[m] = min(max(ci, 0), a.n3[m] - 1);
-        }
-        const float n = a.nrel[((long long)c3[0] * a.n3[1] + c3[1]) * a.n3[2] + c3[2]];
-        const float rr = __fmul_rn(t, rh);
-        col = __fadd_rn(col, __fmul_rn(__fmul_rn(n, n), __fmul_rn(rr, rr)));
-      }
+      // a source clear of the box's faces has every sample of its rays inside the box
+      bool inside = true;
+      for (int m = 0; m < 3; ++m) inside = inside && sf[m] > 0.01f && sf[m] < (float)a.n3[m] - 0.01f;
+      const float col = inside ? march<false>(a, sf, dc, rh, inv, nstep)
+                               : march<true>(a, sf, dc, rh, inv, nstep);
       // R = sum n^2 r^2 dr in SI: (n_ref^2) (hmin^3) col * (rh / nstep)
       const double R = (double)col * ((double)rh * (double)inv) * a.nref * a.nref * hmin * hmin *
                        hmin;
