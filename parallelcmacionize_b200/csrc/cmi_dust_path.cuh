@@ -248,8 +248,9 @@ __global__ void __launch_bounds__(kPathThreads, kMinBlocks)
       }
       waiting = (uint32_t)__popc(__ballot_sync(kFull, status != kRun && status != kExited));
     }
-    // one crossing per lane and turn, until enough more lanes wait
-    const uint32_t enough = min(32u, waiting + kPathTransit);
+    // crossings, until enough more lanes wait (half of those left when they are few)
+    const uint32_t enough =
+        min(32u, waiting + max(1u, min(kPathTransit, (33u - waiting) / 2u)));
     bool over = true;
 #pragma unroll 1
     for (int u = 0; u < kPathStretch; ++u) {

@@ -75,7 +75,10 @@ struct PathParams {
 };
 
 constexpr int kPathFree = 4;      // lane status beyond WalkStatus and kDrop
-constexpr int kPathStretch = 64;  // steps between two looks at the step bound
+constexpr int kPathStretch = 32;  // looks between two checks of the step bound
+// crossings between two looks at the warp (B200, us per iteration at 1 / 2 / 3: stromgren 64^3
+// 349 / 340 / 354, log-normal 128^3 2136 / 2083 / 2151, reemission 687 / 649 / 662)
+constexpr int kPathLook = 2;
 // A warp turns to its lanes at subgrid faces once this many more lanes wait than it
 // could not help, and absorbs and refills once this many lanes do not walk.  B200,
 // us per iteration (stromgren 64^3, 1e6 packets / log-normal 128^3, 1e7): 7 and 8 ->
@@ -951,12 +954,15 @@ __global__ void __launch_bounds__(kPathThreads, kMinBlocks) k_path(const __grid_
       }
       waiting = (uint32_t)__popc(__ballot_sync(kFull, status != kRun && status != kExited));
     }
-    // one crossing per lane and turn, until enough more lanes wait
-    const uint32_t enough = min(32u, waiting + kPathTransit);
+    // crossings, until enough more lanes wait (half of those left when they are few)
+    const uint32_t enough =
+        min(32u, waiting + max(1u, min(kPathTransit, (33u - waiting) / 2u)));
     bool over = true;
 #pragma unroll 1
     for (int u = 0; u < kPathStretch; ++u) {
-      if (status == kRun) status = w.step(prm, sh.geo, tab);
+#pragma unroll
+      for (int k = 0; k < kPathLook; ++k)
+        if (status == kRun) status = w.step(prm, sh.geo, tab);
       if ((uint32_t)__popc(__ballot_sync(kFull, status != kRun)) >= enough) {
         over = false;
         break;
