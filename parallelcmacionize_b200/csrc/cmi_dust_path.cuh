@@ -51,6 +51,8 @@ constexpr uint32_t kDustMaxGenerations = 4096u;
 // lanes whose walk has ended before the warp turns to them (B200, 128^3 / 32^3 above:
 // 10 -> 11.1 / 1.66 ms, 16 -> 10.5 / 1.45, 24 -> 11.4 / 1.34, with 6 CTAs per SM)
 constexpr uint32_t kDustRefill = 16u;
+// lanes at a subgrid face, likewise
+constexpr uint32_t kDustTransit = 12u;
 
 __device__ __forceinline__ void dust_direct(const DustPathParams &prm, DustWalk &w,
                                             const DevGeo &g, const double dir[3]) {
@@ -250,7 +252,7 @@ __global__ void __launch_bounds__(kPathThreads, kMinBlocks)
     }
     // crossings, until enough more lanes wait (half of those left when they are few)
     const uint32_t enough =
-        min(32u, waiting + max(1u, min(kPathTransit, (33u - waiting) / 2u)));
+        min(32u, waiting + max(1u, min(kDustTransit, (33u - waiting) / 2u)));
     bool over = true;
 #pragma unroll 1
     for (int u = 0; u < kPathStretch; ++u) {

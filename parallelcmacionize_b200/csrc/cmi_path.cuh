@@ -22,8 +22,8 @@
 // * The cell faces and subgrid anchors of an instance sit in a shared-memory table;
 //   the entry beyond the last face is a guard (a NaN), so leaving a subgrid is seen in
 //   the face that is loaded anyway.
-// * Lanes at a face, done and free ones wait until several do (kPathTransit,
-//   kPathRefill); packets are emitted 32 at a time into a queue.
+// * Lanes at a face, done and free ones wait until several do (kTransit and kRefill of
+//   the lane state); packets are emitted 32 at a time into a queue.
 //
 // Bound by instruction issue and lane divergence (log-normal 128^3, mixed: 54% of
 // issue slots, 19 of 32 lanes, L1 58% and L2 37% of peak).  Against the wavefront, us
@@ -79,12 +79,6 @@ constexpr int kPathStretch = 32;  // looks between two checks of the step bound
 // crossings between two looks at the warp (B200, us per iteration at 1 / 2 / 3: stromgren 64^3
 // 349 / 340 / 354, log-normal 128^3 2136 / 2083 / 2151, reemission 687 / 649 / 662)
 constexpr int kPathLook = 2;
-// A warp turns to its lanes at subgrid faces once this many more lanes wait than it
-// could not help, and absorbs and refills once this many lanes do not walk.  B200,
-// us per iteration (stromgren 64^3, 1e6 packets / log-normal 128^3, 1e7): 7 and 8 ->
-// 355 / 2133, 10 and 10 -> 335 / 2036, 12 and 14 -> 336 / 2034; with reemission 960,
-// 885, 839 (more lanes wait for the draws).
-constexpr uint32_t kPathTransit = 12, kPathRefill = 12;
 // shared memory a CTA may take: six CTAs (the FP64-geometry build) fit an SM and leave
 // its L1 most of the rest
 constexpr size_t kPathSmemMost = 32768;
@@ -197,6 +191,12 @@ __device__ __forceinline__ uint32_t exit_sides(uint32_t out, const float sg[3]) 
 template <bool kMixed, bool kDefer, bool kTally = true>
 struct PathF {
   using Real = typename std::conditional<kMixed, float, double>::type;
+  // A warp turns to its lanes at subgrid faces once kTransit more lanes wait than it
+  // could not help, and absorbs and refills once kRefill lanes do not walk.  B200, us per
+  // shoot with 12 and 12 / 16 and 6: stromgren 64^3, 1e6 packets 374 / 361, log-normal
+  // 128^3, 1e7 1664 / 1630, 12 uneven instances 3340 / 3260; with reemission, where
+  // more lanes wait for the draws, 644 / 697.
+  static constexpr uint32_t kTransit = kDefer ? 16 : 12, kRefill = kDefer ? 6 : 12;
   double pos[3], d[3], inv[3], face[3];
   uint32_t fi[3];       // shared-memory address of the face ahead
   int sg[3];            // to the next face in bytes: +8 / -8, 0: no motion along the axis
@@ -539,6 +539,8 @@ struct PathF {
 // Lane state of the FP32 cell-unit walk: Walk32's operations.
 template <bool kDefer>
 struct Path32 {
+  // as in PathF; 96 x 80 x 112, 4e6 packets, us per shoot with 12 and 12 / 16 and 6: 1981 / 2014
+  static constexpr uint32_t kTransit = 12, kRefill = 12;
   float p[3], face[3], inv[3], dcs[3];
   float fexit[3];
   float sg[3];          // +1 / -1, 0: no motion along the axis
@@ -905,7 +907,7 @@ __global__ void __launch_bounds__(kPathThreads, kMinBlocks) k_path(const __grid_
     // lanes that are done with their packet, and new packets for them
     const unsigned done = __ballot_sync(kFull, status != kRun);
     uint32_t waiting = (uint32_t)__popc(done);
-    if (waiting >= kPathRefill || done == kFull) {
+    if (waiting >= W::kRefill || done == kFull) {
       if (status == kAbsorbed) {
         w.template absorb<kReemit>(prm, sh.geo);
         cross += (uint32_t)w.steps;
@@ -956,7 +958,7 @@ __global__ void __launch_bounds__(kPathThreads, kMinBlocks) k_path(const __grid_
     }
     // crossings, until enough more lanes wait (half of those left when they are few)
     const uint32_t enough =
-        min(32u, waiting + max(1u, min(kPathTransit, (33u - waiting) / 2u)));
+        min(32u, waiting + max(1u, min(W::kTransit, (33u - waiting) / 2u)));
     bool over = true;
 #pragma unroll 1
     for (int u = 0; u < kPathStretch; ++u) {
