@@ -86,12 +86,12 @@ __global__ void __launch_bounds__(kPathThreads, kMinBlocks)
         reinterpret_cast<const uint32_t *>(prm.path.geo)[i];
   if (lane == 0) sh.job = sh.job_end = sh.q_at = sh.q_n = sh.exhausted = 0u;
   __syncwarp();
-  path_table(table, sh.geo, prm.path.subs, lane);
+  path_table(table, sh, prm.path.subs, 0u, lane);
   __syncwarp();
   if (lane == 0) {
     sh.geo.sigma = 1.;  // the cross section of the dust packets
     DustWalk at;
-    at.at_position(prm.path, 0u, sh, tab, prm.src, prm.src_sub);
+    at.at_position(prm.path, sh, tab, prm.src, prm.src_sub);
   }
   __syncwarp();
   const double never = __longlong_as_double(0x7ff0000000000000ll);
@@ -186,7 +186,7 @@ __global__ void __launch_bounds__(kPathThreads, kMinBlocks)
               }
             }
             dust_direct(prm, w, sh.geo, dir);
-            status = w.reenter(prm.path, 0u, sh, lane, tab, q, 0u);
+            status = w.reenter(prm.path, sh, lane, tab, q, 0u);
           }
         } else {
           status = kPathFree;
@@ -274,7 +274,7 @@ __global__ void __launch_bounds__(kPathThreads, kMinBlocks)
       dl.depth[lane] = __dadd_rn(dl.depth[lane], w.done);
       const double ex = __dadd_rn(w.pos[0], table_at(sh.ci[0][lane]));
       const double ey = __dadd_rn(w.pos[1], table_at(sh.ci[1][lane]));
-      status = w.transit(prm.path, 0u, sh, lane, tab);
+      status = w.transit(prm.path, sh, lane, tab);
       if (status == kPathFree) {  // out of the box
         w.pos[0] = ex;
         w.pos[1] = ey;

@@ -84,15 +84,25 @@ constexpr int kPathLook = 2;
 constexpr size_t kPathSmemMost = 32768;
 constexpr uint32_t kGuardHi = 0x7ff80000u;  // high word of the guard (a NaN)
 
+// What the turn at a subgrid face needs of an axis.
+struct alignas(16) PathAxis {
+  double inv_cs;
+  uint32_t low;   // address in the table of the face behind cell 0, 12 bytes on
+  uint32_t span;  // cells of a subgrid
+  int32_t sub_stride, jump;
+};
+
 // Per-warp shared memory: the instance's geometry, the state of a packet at the
 // current source, a queue of up to 32 emitted packets, then the table.
 struct PathShared {
   DevGeo geo;
+  PathAxis axis[3];
   double q_dir[3][32], q_inv[3][32], q_tau[32];
   double src_pos[3];       // relative to the subgrid's anchor (FP32: in cells)
   int32_t src_idx[3];
   uint32_t src_c[3];
   uint32_t src_sub, src_cell, src_toff, src_out;
+  uint32_t copy_base;      // tally word of a copied cell: field cell + first copied cell + this
   // per lane, what only the turn at a subgrid face needs
   uint32_t ci[3][32];      // subgrid anchors (FP64 geometry: table addresses; FP32: coordinates)
   uint32_t sub[32];        // subgrid of the instance
@@ -105,9 +115,15 @@ struct PathShared {
   uint32_t absorbed[32], escaped[32], reemitted[32], most[32];
 };
 
-// the face and anchor table of an instance, filled by one warp
-__device__ __forceinline__ void path_table(double *tab, const DevGeo &g, const DevSubgrid *subs,
-                                           int lane) {
+// The face and anchor table of the warp's instance, and what follows from it for a warp
+// that adds to tally copy `copy`; all lanes.
+__device__ __forceinline__ void path_table(double *tab, PathShared &sh, const DevSubgrid *subs,
+                                           uint32_t copy, int lane) {
+  const DevGeo &g = sh.geo;
+  if (lane < 3)
+    sh.axis[lane] = {g.inv_cs[lane], smem_addr(tab) + 12u + 8u * (uint32_t)g.face_off[lane],
+                     (uint32_t)g.n[lane], g.sub_stride[lane], g.jump[lane]};
+  if (lane == 0) sh.copy_base = copy * g.padded - g.first_cell;
   const double guard = __hiloint2double((int)kGuardHi, 0);
   if (lane == 0) tab[g.inf_off] = __longlong_as_double(0x7ff0000000000000ll);
   for (int a = 0; a < 3; ++a) {
@@ -123,10 +139,10 @@ __device__ __forceinline__ void path_table(double *tab, const DevGeo &g, const D
 }
 
 // offset of this warp's tally copy of a subgrid (0: no copies, the field itself)
-__device__ __forceinline__ uint32_t tally_offset(const PathParams &prm, const DevGeo &g,
-                                                 uint32_t sub, uint32_t copy) {
-  const uint32_t hot = __ldg(prm.hot + g.first_sub + sub);
-  return hot ? hot + copy * g.padded - (g.first_cell + sub * g.padded) : 0u;
+__device__ __forceinline__ uint32_t tally_offset(const PathParams &prm, const PathShared &sh,
+                                                 uint32_t sub) {
+  const uint32_t hot = __ldg(prm.hot + sh.geo.first_sub + sub);
+  return hot ? hot + (sh.copy_base - sub * sh.geo.padded) : 0u;
 }
 
 __device__ __forceinline__ double table_at(uint32_t byte) {
@@ -257,7 +273,7 @@ struct PathF {
     }
     return out;
   }
-  __device__ __forceinline__ int settle(const PathParams &prm, uint32_t copy, const PathShared &sh, int lane,
+  __device__ __forceinline__ int settle(const PathParams &prm, const PathShared &sh, int lane,
                                         uint32_t tab, const int idx[3], uint32_t out) {
     const DevGeo &g = sh.geo;
     const uint32_t sub = sh.sub[lane];
@@ -266,7 +282,7 @@ struct PathF {
     if (out) return kExited;
     cell = g.first_cell + sub * g.padded +
            (uint32_t)(idx[0] * g.stride[0] + idx[1] * g.stride[1] + idx[2]);
-    toff = kTally ? tally_offset(prm, g, sub, copy) : 0u;
+    toff = kTally ? tally_offset(prm, sh, sub) : 0u;
 #pragma unroll
     for (int a = 0; a < 3; ++a) ahead(g, tab, a, idx[a]);
     if (!kDefer) opacity(prm, lk, lx);
@@ -274,12 +290,11 @@ struct PathF {
   }
 
   // the state of a packet at the source, shared by the warp
-  __device__ __forceinline__ void at_source(const PathParams &prm, uint32_t copy, PathShared &sh,
+  __device__ __forceinline__ void at_source(const PathParams &prm, PathShared &sh,
                                             uint32_t tab, const DevSource &S) {
-    at_position(prm, copy, sh, tab, S.position, S.subgrid - sh.geo.first_sub);
+    at_position(prm, sh, tab, S.position, S.subgrid - sh.geo.first_sub);
   }
-  __device__ __forceinline__ void at_position(const PathParams &prm, uint32_t copy,
-                                              PathShared &sh, uint32_t tab,
+  __device__ __forceinline__ void at_position(const PathParams &prm, PathShared &sh, uint32_t tab,
                                               const double position[3], uint32_t sub) {
     const DevGeo &g = sh.geo;
     int idx[3];
@@ -297,7 +312,7 @@ struct PathF {
     sh.src_sub = sub;
     sh.src_cell = g.first_cell + sub * g.padded +
                   (uint32_t)(idx[0] * g.stride[0] + idx[1] * g.stride[1] + idx[2]);
-    sh.src_toff = kTally ? tally_offset(prm, g, sub, copy) : 0u;
+    sh.src_toff = kTally ? tally_offset(prm, sh, sub) : 0u;
     sh.src_out = out;
   }
   __device__ __forceinline__ int start(const PathParams &prm, PathShared &sh, int lane,
@@ -320,18 +335,18 @@ struct PathF {
 
   // Entry into the subgrid on the other side of the faces in `in` (bit a: axis a, bit
   // 3 + a: upwards) at the absolute position q, with every index found afresh.
-  __device__ __forceinline__ int reenter(const PathParams &prm, uint32_t copy, PathShared &sh,
+  __device__ __forceinline__ int reenter(const PathParams &prm, PathShared &sh,
                                          int lane, uint32_t tab, const double q[3], uint32_t in) {
     double anchor[3];
     int idx[3];
 #pragma unroll
     for (int a = 0; a < 3; ++a) anchor[a] = table_at(sh.ci[a][lane]);
     const uint32_t out = locate(sh.geo, anchor, q, in, idx);
-    return settle(prm, copy, sh, lane, tab, idx, out);
+    return settle(prm, sh, lane, tab, idx, out);
   }
 
   // a packet found outside the subgrid's index range at entry moves on at once
-  __device__ __forceinline__ int pass_on(const PathParams &prm, uint32_t copy, PathShared &sh,
+  __device__ __forceinline__ int pass_on(const PathParams &prm, PathShared &sh,
                                          int lane, uint32_t tab) {
     const DevGeo &g = sh.geo;
     double q[3];
@@ -346,47 +361,52 @@ struct PathF {
       outside = outside || (uint32_t)__double2hiint(table_at(sh.ci[a][lane])) == kGuardHi;
     }
     if (outside) return kPathFree;
-    return reenter(prm, copy, sh, lane, tab, q, ex);
+    return reenter(prm, sh, lane, tab, q, ex);
   }
 
   // Across the face(s) it left by into the next subgrid: pos + anchor of this one -
   // anchor of the next, remaining depth, start index.  kPathFree: out of the box.
-  __device__ __forceinline__ int transit(const PathParams &prm, uint32_t copy, PathShared &sh,
+  __device__ __forceinline__ int transit(const PathParams &prm, PathShared &sh,
                                          int lane, uint32_t tab) {
-    const DevGeo &g = sh.geo;
     target = kMixed ? (Real)__fsub_rn((float)target, (float)done)
                     : (Real)__dsub_rn((double)target, (double)done);
     done = (Real)0;
-    if (steps == 0) return pass_on(prm, copy, sh, lane, tab);
+    if (steps == 0) return pass_on(prm, sh, lane, tab);
     steps = 0;
-    double q[3];
+    double q[3], anchor[3];
     bool outside = false, same = true;
-    uint32_t sub = sh.sub[lane];
+    uint32_t sub = sh.sub[lane], ci[3];
+    int hop[3];
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-      uint32_t ci = sh.ci[a][lane];
-      q[a] = __dadd_rn(pos[a], table_at(ci));
-      const bool off = (uint32_t)__double2hiint(face[a]) == kGuardHi;
-      if (off) {
-        ci += (uint32_t)sg[a];
-        sh.ci[a][lane] = ci;
-        sub += (uint32_t)(sg[a] > 0 ? g.sub_stride[a] : -g.sub_stride[a]);
-        cell += (uint32_t)(sg[a] > 0 ? g.jump[a] : -g.jump[a]);
-        fi[a] -= (uint32_t)(sg[a] * g.n[a]);
-      }
-      const double anchor = table_at(ci);
-      outside = outside || (uint32_t)__double2hiint(anchor) == kGuardHi;
-      pos[a] = __dsub_rn(q[a], anchor);
+      ci[a] = sh.ci[a][lane];
+      q[a] = __dadd_rn(pos[a], table_at(ci[a]));
+      hop[a] = (uint32_t)__double2hiint(face[a]) == kGuardHi ? sg[a] : 0;  // 8 bytes up or down
+      ci[a] += (uint32_t)hop[a];
+      anchor[a] = table_at(ci[a]);
+    }
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      const PathAxis &A = sh.axis[a];
+      sh.ci[a][lane] = ci[a];
+      const int one = hop[a] >> 3;
+      sub += (uint32_t)(one * A.sub_stride);
+      cell += (uint32_t)(one * A.jump);
+      fi[a] -= (uint32_t)hop[a] * A.span;
+      outside = outside || (uint32_t)__double2hiint(anchor[a]) == kGuardHi;
+      pos[a] = __dsub_rn(q[a], anchor[a]);
       // the start index of an axis it did not leave by is the present one but for
-      // rounding; an axis it left by starts at the first cell behind the face
-      const int idx = __double2int_rz(__dmul_rn(pos[a], g.inv_cs[a]));
-      same = same && (off || fi[a] - (uint32_t)(sg[a] >> 1) ==
-                                 tab + 12u + 8u * (uint32_t)(g.face_off[a] + idx));
+      // rounding; an axis it left by starts at the first cell behind the face.  The low
+      // word of the sum is the index rounded down; below 0, where truncation
+      // differs, it matches no cell and the entry is found afresh.
+      const int idx = __double2loint(__dadd_rd(__dmul_rn(pos[a], A.inv_cs), 6755399441055744.));
+      same = same && (hop[a] != 0 ||
+                      fi[a] - (uint32_t)(sg[a] >> 1) == A.low + 8u * (uint32_t)idx);
     }
     if (outside) return kPathFree;
     sh.sub[lane] = sub;
     if (same) {
-      if (kTally) toff = tally_offset(prm, g, sub, copy);
+      if (kTally) toff = tally_offset(prm, sh, sub);
       // the guard on the axes it left by: read again
 #pragma unroll
       for (int a = 0; a < 3; ++a) face[a] = table_at(fi[a]);
@@ -397,11 +417,11 @@ struct PathF {
 #pragma unroll
     for (int a = 0; a < 3; ++a)
       if ((uint32_t)__double2hiint(face[a]) == kGuardHi) in |= (sg[a] > 0 ? 9u : 1u) << a;
-    return reenter(prm, copy, sh, lane, tab, q, in);
+    return reenter(prm, sh, lane, tab, q, in);
   }
 
   // back to the absorption point with a new direction and depth
-  __device__ __forceinline__ int reemit(const PathParams &prm, uint32_t copy, const PathShared &sh, int lane,
+  __device__ __forceinline__ int reemit(const PathParams &prm, const PathShared &sh, int lane,
                                         uint32_t tab, const double rd[4]) {
     const DevGeo &g = sh.geo;
     double q[3], anchor[3];
@@ -414,7 +434,7 @@ struct PathF {
     }
     depth(rd[3]);
     const uint32_t out = locate(g, anchor, q, 0u, idx);
-    return settle(prm, copy, sh, lane, tab, idx, out);
+    return settle(prm, sh, lane, tab, idx, out);
   }
   __device__ __forceinline__ void reemit_counter(const PathShared &sh, int lane, uint32_t tab,
                                                  uint32_t h[3]) const {
@@ -591,7 +611,7 @@ struct Path32 {
     }
     return out;
   }
-  __device__ __forceinline__ int settle(const PathParams &prm, uint32_t copy, const PathShared &sh, int lane,
+  __device__ __forceinline__ int settle(const PathParams &prm, const PathShared &sh, int lane,
                                         const int idx[3], uint32_t out) {
     const DevGeo &g = sh.geo;
     const uint32_t sub = sh.sub[lane];
@@ -602,10 +622,10 @@ struct Path32 {
     if (out) return kExited;
     cell = g.first_cell + sub * g.padded +
            (uint32_t)(idx[0] * g.stride[0] + idx[1] * g.stride[1] + idx[2]);
-    toff = tally_offset(prm, g, sub, copy);
+    toff = tally_offset(prm, sh, sub);
     return kRun;
   }
-  __device__ __forceinline__ void at_source(const PathParams &prm, uint32_t copy, PathShared &sh,
+  __device__ __forceinline__ void at_source(const PathParams &prm, PathShared &sh,
                                             uint32_t, const DevSource &S) {
     const DevGeo &g = sh.geo;
     const uint32_t sub = S.subgrid - g.first_sub;
@@ -621,7 +641,7 @@ struct Path32 {
     sh.src_sub = sub;
     sh.src_cell = g.first_cell + sub * g.padded +
                   (uint32_t)(idx[0] * g.stride[0] + idx[1] * g.stride[1] + idx[2]);
-    sh.src_toff = tally_offset(prm, g, sub, copy);
+    sh.src_toff = tally_offset(prm, sh, sub);
     sh.src_out = out;
   }
   __device__ __forceinline__ int start(const PathParams &, PathShared &sh, int lane, uint32_t) {
@@ -639,7 +659,7 @@ struct Path32 {
     return ex ? kExited : kRun;
   }
   // the exit coordinate is 0 or n, so re-anchoring is exact
-  __device__ __forceinline__ int transit(const PathParams &prm, uint32_t copy, PathShared &sh, int lane,
+  __device__ __forceinline__ int transit(const PathParams &prm, PathShared &sh, int lane,
                                          uint32_t) {
     const DevGeo &g = sh.geo;
     const bool crossed = steps > 0;
@@ -672,13 +692,13 @@ struct Path32 {
         face[a] = off ? (sg[a] > 0 ? 1.f : (float)(g.n[a] - 1)) : face[a];
         cell += off ? (uint32_t)(sg[a] > 0.f ? g.jump[a] : -g.jump[a]) : 0u;
       }
-      toff = tally_offset(prm, g, sub, copy);
+      toff = tally_offset(prm, sh, sub);
       return 0.f < target ? kRun : kAbsorbed;
     }
     const uint32_t out = locate(g, ex, idx);
-    return settle(prm, copy, sh, lane, idx, out);
+    return settle(prm, sh, lane, idx, out);
   }
-  __device__ __forceinline__ int reemit(const PathParams &prm, uint32_t copy, const PathShared &sh, int lane,
+  __device__ __forceinline__ int reemit(const PathParams &prm, const PathShared &sh, int lane,
                                         uint32_t, const double rd[4]) {
     const DevGeo &g = sh.geo;
     int idx[3];
@@ -686,7 +706,7 @@ struct Path32 {
     for (int a = 0; a < 3; ++a) direction(g, a, rd[a], inverse(g, a, rd[a]));
     depth(rd[3]);
     const uint32_t out = locate(g, 0u, idx);
-    return settle(prm, copy, sh, lane, idx, out);
+    return settle(prm, sh, lane, idx, out);
   }
   __device__ __forceinline__ void reemit_counter(const PathShared &sh, int lane, uint32_t,
                                                  uint32_t h[3]) const {
@@ -849,7 +869,7 @@ __device__ __noinline__ void path_emit(const PathParams &prm, PathShared &sh, do
         reinterpret_cast<uint32_t *>(&sh.geo)[i] =
             reinterpret_cast<const uint32_t *>(prm.geo + inst)[i];
       __syncwarp();
-      path_table(table, sh.geo, prm.subs, lane);
+      path_table(table, sh, prm.subs, copy, lane);
       __syncwarp();
     }
     if (lane == 0) {
@@ -858,7 +878,7 @@ __device__ __noinline__ void path_emit(const PathParams &prm, PathShared &sh, do
       sh.src_begin = (uint32_t)prm.src_first[s];
       sh.src_end = (uint32_t)prm.src_first[s + 1];
       W at;
-      at.at_source(prm, copy, sh, smem_addr(table), prm.src[s]);
+      at.at_source(prm, sh, smem_addr(table), prm.src[s]);
     }
     __syncwarp();
   }
@@ -921,7 +941,7 @@ __global__ void __launch_bounds__(kPathThreads, kMinBlocks) k_path(const __grid_
                                sh.again[lane], sh.geo.reemission, rd)) {
             ++sh.reemitted[lane];
             ++sh.again[lane];
-            status = w.reemit(prm, copy, sh, lane, tab, rd);
+            status = w.reemit(prm, sh, lane, tab, rd);
           }
         }
         if (status == kPathFree) {
@@ -979,7 +999,7 @@ __global__ void __launch_bounds__(kPathThreads, kMinBlocks) k_path(const __grid_
     if (status == kExited) {
       cross += (uint32_t)w.steps;
       ++trans;
-      status = w.transit(prm, copy, sh, lane, tab);
+      status = w.transit(prm, sh, lane, tab);
       if (kReemit) sh.again[lane] = 0u;
       const uint32_t v = sh.visits[lane] + 1u;
       sh.visits[lane] = v;
