@@ -1038,6 +1038,8 @@ constexpr int kWgradThreads = kWgradWarps * 32;
 constexpr int kUnitCols = 48;             // one unit's accumulator: taps dx = -1, 0, 1 x 16
 constexpr int kWgradUnitsPerCta = 10;     // 10 x 48 <= 512 TMEM columns
 constexpr int kWgMaxBufs = 4;             // tile buffers in flight at most
+constexpr size_t kWgStaticSmem = 2048;    // static shared memory of a CTA and what the
+                                          // system keeps of it
 
 // dy of a tile with one extra voxel row on either side in y, 16 channels per
 // 32-byte voxel row (32-byte swizzle), x fastest:
@@ -1105,7 +1107,6 @@ __global__ void __launch_bounds__(kWgradThreads) k_conv3_wgrad_tc(
   uint64_t *empty = full + kWgMaxBufs;  // the MMAs done (1) and dy summed (4 warps)
   uint64_t *drain = empty + kWgMaxBufs;  // the MMAs in flight when the CTA ends
   uint32_t *tslot = reinterpret_cast<uint32_t *>(drain + 1);
-  __shared__ float s_db[128];  // the CTA's bias-gradient sums
   __shared__ int s_abort;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int nunits = 3 * ncc * a.nchunk;
@@ -1115,7 +1116,6 @@ __global__ void __launch_bounds__(kWgradThreads) k_conv3_wgrad_tc(
   const int nmine = (blockIdx.x < tiles && nunit > 0)
                         ? (tiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
 
-  for (int c = tid; c < 128; c += kWgradThreads) s_db[c] = 0.f;
   if (tid == 0) {
     s_abort = 0;
     for (int s = 0; s < a.nbuf; ++s) {
@@ -1139,6 +1139,13 @@ __global__ void __launch_bounds__(kWgradThreads) k_conv3_wgrad_tc(
   volatile int *abort = &s_abort;
   const uint32_t bytes = (uint32_t)((size_t)ncc * D::kCopies * D::kCopyBytes +
                                     (size_t)a.nchunk * T::kCopies * T::kCopyBytes);
+  // bias gradient: dy[v][co] summed over the CTA's tiles (the first group's
+  // CTAs).  The 16-byte halves of the dy rows (8 channels each; 2 per 16-channel
+  // chunk) are spread over the 128 threads of warps 0-3: thread t reads half
+  // p = t % pairs of rows t / pairs, + 128 / pairs, ...
+  const bool sum = a.db && blockIdx.y == 0;  // CTA-uniform
+  const int pairs = 2 * ncc, tpp = 128 / pairs;
+  float bsum[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 
   if (warp == 4 && lane == 0) {
     int issued = 0;
@@ -1209,15 +1216,9 @@ __global__ void __launch_bounds__(kWgradThreads) k_conv3_wgrad_tc(
     commit_el(drain);
     mbar_wait(drain, 0, a.err);
   } else if (warp < 4) {
-    // bias gradient: dy[v][co] summed over the CTA's tiles (the first group's
-    // CTAs; the others only release the buffers).  The 16-byte halves of the
-    // dy rows (8 channels each; 2 per 16-channel chunk) are spread over the
-    // 128 threads: thread t reads half p = t % pairs of rows t / pairs,
-    // + 128 / pairs, ...; its 8 sums go to shared memory at the end.
-    const bool sum = a.db && blockIdx.y == 0;  // CTA-uniform
-    const int pairs = 2 * ncc, tpp = 128 / pairs, p = tid % pairs, r0 = tid / pairs;
+    // bias sums, and the release of the buffers
+    const int p = tid % pairs, r0 = tid / pairs;
     const bool mine = sum && r0 < tpp;
-    float bsum[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     for (int i = 0; i < nmine; ++i) {
       const int b = i % a.nbuf;
       bool ok0 = true;
@@ -1240,15 +1241,27 @@ __global__ void __launch_bounds__(kWgradThreads) k_conv3_wgrad_tc(
         asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&empty[b]))
                      : "memory");
     }
-    if (mine) {
-#pragma unroll
-      for (int e = 0; e < 8; ++e) atomicAdd(&s_db[p * 8 + e], bsum[e]);
-    }
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  if (a.db && blockIdx.y == 0 && nmine > 0 && tid < a.cout_real) atomicAdd(&a.db[tid], s_db[tid]);
+  if (sum && nmine > 0 && !*abort) {
+    // The threads' sums meet in the first tile buffer (every copy and MMA is done).
+    // FP32 atomics in shared memory are retry loops: 64 threads to an address took
+    // 8 us of a launch.
+    float *part = reinterpret_cast<float *>(sm);
+    if (warp < 4) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) part[e * 128 + tid] = bsum[e];
+    }
+    __syncthreads();
+    if (tid < a.cout_real) {
+      const float *q = part + (tid & 7) * 128 + (tid >> 3);
+      float v = 0.f;
+      for (int k = 0; k < tpp; ++k) v += q[k * pairs];
+      atomicAdd(&a.db[tid], v);
+    }
+  }
   if (a.part && warp < 2 && (nmine == 0 || *abort)) {
     // no tiles: this CTA's share of the sums is zero
     const int lrow = warp * 32 + lane;
@@ -2439,16 +2452,18 @@ int wgrad_t(cmi_unet *u, const Slice &x, const Slice &dy, float *dw, float *db,
     return (std::max(nbuf * buf, reach_end) + 127) / 128 * 128;
   };
   auto smem_for = [&](int nbuf) { return 1024 + bars_at(nbuf) + 128; };
-  // as many tile buffers (up to kWgMaxBufs) as leave room for the CTAs per SM
-  // that the tensor memory allows
-  const int tmem_ctas = std::max(1, (int)(512 / a.tmem_cols));
-  const size_t cap = std::min<size_t>((size_t)optin, 233472 / tmem_ctas - 2048);
-  a.nbuf = smem_for(2) <= (size_t)optin ? 2 : 1;  // fewer CTAs per SM before one buffer
-  for (int nb = kWgMaxBufs; nb > 2; --nb)
-    if (smem_for(nb) <= cap) {
-      a.nbuf = nb;
-      break;
-    }
+  // CTAs per SM that the tensor memory allows (the occupancy query answers one for
+  // this kernel) and tile buffers (kWgMaxBufs at most): the most buffers per SM
+  int per_sm = 1;
+  a.nbuf = 1;
+  for (int c = 1; c <= (int)(512 / a.tmem_cols); ++c)
+    for (int nb = 2; nb <= kWgMaxBufs; ++nb)
+      if (smem_for(nb) <= (size_t)optin &&
+          c * (smem_for(nb) + kWgStaticSmem) <= (size_t)optin + kWgStaticSmem &&
+          c * nb >= per_sm * a.nbuf) {
+        per_sm = c;
+        a.nbuf = nb;
+      }
   a.bar_off = (int)bars_at(a.nbuf);
   const size_t smem = smem_for(a.nbuf);
   if (smem > (size_t)optin)
@@ -2456,11 +2471,6 @@ int wgrad_t(cmi_unet *u, const Slice &x, const Slice &dy, float *dw, float *db,
   // the whole opt-in size, the same for every launch (see xf_launch)
   UN_CUDA(cudaFuncSetAttribute(k_conv3_wgrad_tc<TY>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                optin));
-  int per_sm = 0;
-  UN_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_conv3_wgrad_tc<TY>,
-                                                        kWgradThreads, smem));
-  // TMEM: at most 512 columns per SM
-  per_sm = std::max(1, std::min(per_sm, (int)(512 / a.tmem_cols)));
   int sms = 0, dev = 0;
   UN_CUDA(cudaGetDevice(&dev));
   UN_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
