@@ -272,6 +272,41 @@ __device__ __forceinline__ Bf8 load8(const bf16 *p) {
   }
   return r;
 }
+// 16 BF16 channels of a voxel (32 bytes); wide: 32-byte aligned, one access
+struct Row16 {
+  uint32_t w[8];
+  __device__ __forceinline__ __nv_bfloat162 pair(int e) const {
+    return *reinterpret_cast<const __nv_bfloat162 *>(&w[e / 2]);
+  }
+  __device__ __forceinline__ void set(int e, __nv_bfloat162 v) {
+    w[e / 2] = *reinterpret_cast<const uint32_t *>(&v);
+  }
+};
+__device__ __forceinline__ Row16 load_row16(const bf16 *p, bool wide) {
+  Row16 r;
+  if (wide) {
+    asm volatile("ld.global.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(r.w[0]), "=r"(r.w[1]), "=r"(r.w[2]), "=r"(r.w[3]), "=r"(r.w[4]),
+                   "=r"(r.w[5]), "=r"(r.w[6]), "=r"(r.w[7])
+                 : "l"(p));
+  } else {
+    const uint4 a = reinterpret_cast<const uint4 *>(p)[0], b = reinterpret_cast<const uint4 *>(p)[1];
+    r.w[0] = a.x, r.w[1] = a.y, r.w[2] = a.z, r.w[3] = a.w;
+    r.w[4] = b.x, r.w[5] = b.y, r.w[6] = b.z, r.w[7] = b.w;
+  }
+  return r;
+}
+__device__ __forceinline__ void store_row16(bf16 *p, const Row16 &r, bool wide) {
+  if (wide) {
+    asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(r.w[0]),
+                 "r"(r.w[1]), "r"(r.w[2]), "r"(r.w[3]), "r"(r.w[4]), "r"(r.w[5]), "r"(r.w[6]),
+                 "r"(r.w[7])
+                 : "memory");
+  } else {
+    reinterpret_cast<uint4 *>(p)[0] = make_uint4(r.w[0], r.w[1], r.w[2], r.w[3]);
+    reinterpret_cast<uint4 *>(p)[1] = make_uint4(r.w[4], r.w[5], r.w[6], r.w[7]);
+  }
+}
 __device__ __forceinline__ void store8(bf16 *p, const Bf8 &r) {
   uint4 q;
   __nv_bfloat162 *h = reinterpret_cast<__nv_bfloat162 *>(&q);
@@ -306,6 +341,7 @@ struct ConvArgs {
   float slope;
   const bf16 *gate;      // input-gradient convolutions: out *= leaky'(gate) (may be null)
   int gate_ctot, gate_c0;
+  bool wide;             // k_conv3_xf: rows of out and gate start on 32 bytes
   uint32_t *err;
 };
 constexpr int kConvWarps = 6;               // 0-3 epilogue, 4 loads, 5 MMAs
@@ -656,7 +692,9 @@ struct XTile {
 // combine the x taps, add bias, apply the activation or the derivative gate
 // and store.
 constexpr int kMaxInBufs = 8;
-constexpr int kXfEpiWarps = 8;                      // two per quarter of the TMEM lanes
+// epilogue warps, four per quarter of the TMEM lanes (training step, 64^3 x 8, with two,
+// three, four: 2256, 2242, 2203 us; with 16-byte rows 2222)
+constexpr int kXfEpiWarps = 16;
 constexpr int kXfThreads = (kXfEpiWarps + 2) * 32;  // + loads + MMAs
 // tcgen05.mma and tcgen05.commit issued by one elected lane of a converged warp:
 // the x-folded kernel's MMA role runs its loops on the whole warp, whose
@@ -925,7 +963,7 @@ __global__ void __launch_bounds__(kXfThreads, 1) k_conv3_xf(const __grid_constan
       int x0, y0, z0, n;
       T::origin(blockIdx.x + i * gridDim.x, a.dims, x0, y0, z0, n);
       // row r = u (16 x 8, x fastest); outputs at u columns 1 .. 14 inside the grid.
-      // Warps q and q + 4 read TMEM lanes 32 q .. 32 q + 31 and share the
+      // Warps q, q + 4, ... read TMEM lanes 32 q .. 32 q + 31 and share the
       // (sub-tile, 16-channel group) items of the tile between them.
       const int q = warp & 3, r = q * 32 + lane, ux = r & 15;
       const int vx = x0 + ux, vy = y0 + (r >> 4);
@@ -961,36 +999,33 @@ __global__ void __launch_bounds__(kXfThreads, 1) k_conv3_xf(const __grid_constan
           }
           if (valid) {
             bf16 *dst = a.out + vox * a.out_ctot + a.out_c0 + j;
-            float gy[16];
-            if (a.gate) {
-              const bf16 *gp = a.gate + vox * a.gate_ctot + a.gate_c0 + j;
-              const Bf8 g0 = load8(gp), g1 = load8(gp + 8);
-#pragma unroll
-              for (int e = 0; e < 8; ++e) {
-                gy[e] = g0.v[e];
-                gy[e + 8] = g1.v[e];
-              }
-            }
+            Row16 gy;
+            if (a.gate) gy = load_row16(a.gate + vox * a.gate_ctot + a.gate_c0 + j, a.wide);
             // leaky ReLU as max(x, slope x): the same for 0 <= slope < 1
-            __align__(16) __nv_bfloat162 o[8];
+            Row16 o;
 #pragma unroll
-            for (int e = 0; e < 16; e += 2) {
-              float x0 = f[e] + sbias[j + e], x1 = f[e + 1] + sbias[j + e + 1];
+            for (int e = 0; e < 16; e += 4) {
+              const float4 bias = *reinterpret_cast<const float4 *>(sbias + j + e);
+              float x[4] = {f[e] + bias.x, f[e + 1] + bias.y, f[e + 2] + bias.z,
+                            f[e + 3] + bias.w};
               if (a.act) {
-                x0 = fmaxf(x0, x0 * a.slope);
-                x1 = fmaxf(x1, x1 * a.slope);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) x[k] = fmaxf(x[k], x[k] * a.slope);
               }
               if (a.gate) {
-                x0 = __bfloat162float(__float2bfloat16_rn(x0));
-                x1 = __bfloat162float(__float2bfloat16_rn(x1));
-                if (!(gy[e] > 0.f)) x0 *= a.slope;
-                if (!(gy[e + 1] > 0.f)) x1 *= a.slope;
+#pragma unroll
+                for (int k = 0; k < 4; k += 2) {
+                  const float2 g = __bfloat1622float2(gy.pair(e + k));
+                  x[k] = __bfloat162float(__float2bfloat16_rn(x[k]));
+                  x[k + 1] = __bfloat162float(__float2bfloat16_rn(x[k + 1]));
+                  if (!(g.x > 0.f)) x[k] *= a.slope;
+                  if (!(g.y > 0.f)) x[k + 1] *= a.slope;
+                }
               }
-              o[e / 2] = __floats2bfloat162_rn(x0, x1);
+              o.set(e, __floats2bfloat162_rn(x[0], x[1]));
+              o.set(e + 2, __floats2bfloat162_rn(x[2], x[3]));
             }
-            uint4 *d4 = reinterpret_cast<uint4 *>(dst);
-            d4[0] = reinterpret_cast<const uint4 *>(o)[0];
-            d4[1] = reinterpret_cast<const uint4 *>(o)[1];
+            store_row16(dst, o, a.wide);
           }
         }
       }
@@ -2329,6 +2364,10 @@ int xf_launch(cmi_unet *u, const Slice &in, const bf16 *wpack, const float *bias
     a.gate_ctot = gate->ctot;
     a.gate_c0 = gate->c0;
   }
+  auto rows32 = [](const Slice &r) {
+    return reinterpret_cast<uintptr_t>(r.base) % 32 == 0 && r.ctot % 16 == 0 && r.c0 % 16 == 0;
+  };
+  a.wide = rows32(out) && (!gate || rows32(*gate));
   a.err = u->d_err;
   a.nbuf = p.nbuf;
   a.wstages = p.wstages;
