@@ -51,8 +51,8 @@ constexpr uint32_t kDustMaxGenerations = 4096u;
 // lanes whose walk has ended before the warp turns to them (B200, 128^3 / 32^3 above:
 // 10 -> 11.1 / 1.66 ms, 16 -> 10.5 / 1.45, 24 -> 11.4 / 1.34, with 6 CTAs per SM)
 constexpr uint32_t kDustRefill = 16u;
-// lanes at a subgrid face, likewise
-constexpr uint32_t kDustTransit = 12u;
+// lanes at a subgrid face, likewise (8 / 12 / 16 / 20: 9932 / 9735 / 9680 / 9685 us)
+constexpr uint32_t kDustTransit = 16u;
 
 __device__ __forceinline__ void dust_direct(const DustPathParams &prm, DustWalk &w,
                                             const DevGeo &g, const double dir[3]) {

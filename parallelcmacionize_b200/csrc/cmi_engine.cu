@@ -147,6 +147,7 @@ struct cmi_context {
   bool tables_fit = false;  // path_table fits, whatever carries the iterations
   DevGeo *d_geo = nullptr;
   unsigned long long *d_tally = nullptr;
+  double2 *d_pair = nullptr;  // n_H and x_H side by side (dust)
   uint32_t *d_hot = nullptr;   // per subgrid: first cell of its tally copies, 0: none
   uint32_t copies = 1;
   size_t tally_words = 0, tally_need = 0;
@@ -306,6 +307,7 @@ int ensure_capacity(cmi_context *c, uint64_t packets) {
 int ensure_stage(cmi_context *c, size_t bytes) {
   if (bytes <= c->stage_bytes) return CMI_OK;
   dev_free(c->d_stage);
+  c->stage_bytes = 0;
   CMI_CUDA(cudaMalloc(&c->d_stage, bytes));
   c->stage_bytes = bytes;
   return CMI_OK;
@@ -425,6 +427,16 @@ int ensure_tally(cmi_context *c) {
   c->tally_words = c->tally_need;
   CMI_CUDA(cudaMemsetAsync(c->d_tally, 0, sizeof(unsigned long long) * c->tally_words, c->stream));
   return CMI_OK;
+}
+
+// the fields side by side for the dust walks (16 bytes per cell, made at the first dust
+// run); false: no memory for them
+bool ensure_pair(cmi_context *c) {
+  if (!c->d_pair && cudaMalloc(&c->d_pair, sizeof(double2) * c->total_padded) != cudaSuccess) {
+    cudaGetLastError();
+    c->d_pair = nullptr;
+  }
+  return c->d_pair != nullptr;
 }
 
 // Upload instance + source tables (after sources or budgets change).
@@ -1305,6 +1317,7 @@ int cmi_destroy(cmi_context *c) {
   dev_free(c->d_J);
   dev_free(c->d_geo);
   dev_free(c->d_tally);
+  dev_free(c->d_pair);
   dev_free(c->d_hot);
   dev_free(c->d_kappa);
   dev_free(c->d_src_count);
@@ -2046,8 +2059,11 @@ int dust_by_paths(cmi_context *c, int32_t instance, uint32_t n, uint64_t seed, u
   DustPathParams p{};
   p.path.geo = c->d_geo + instance;
   p.path.subs = c->d_sub;
-  p.path.nH = c->d_nH;
-  p.path.xH = c->d_xH;
+  const HostInstance &I = c->inst[instance];
+  k_pair<<<field_grid(I), 256, 0, c->stream>>>(c->d_sub, I.first_sub, c->d_nH, c->d_xH,
+                                               c->d_pair);
+  CMI_CUDA(cudaGetLastError());
+  p.path.nx = c->d_pair;
   p.path.table = c->path_table;
   p.n = n;
   p.counters = reinterpret_cast<unsigned long long *>(c->d_stage);
@@ -2059,7 +2075,7 @@ int dust_by_paths(cmi_context *c, int32_t instance, uint32_t n, uint64_t seed, u
   p.src_sub = src_sub;
   for (int a = 0; a < 3; ++a) p.src[a] = source[a];
   p.albedo = albedo;
-  const double *box = c->inst[instance].desc.box;
+  const double *box = I.desc.box;
   p.x0 = box[0];
   p.wx = box[3];
   p.y0 = box[1];
@@ -2161,7 +2177,7 @@ extern "C" int cmi_dust_run(cmi_context *c, int32_t instance, uint64_t num_photo
   const size_t npix = (size_t)npix_x * npix_y;
   const uint32_t src_sub =
       (uint32_t)((si[0] * I.desc.num_subgrid[1] + si[1]) * I.desc.num_subgrid[2] + si[2]);
-  if (c->tables_fit)
+  if (c->tables_fit && ensure_pair(c))
     return dust_by_paths(c, instance, n, seed, iteration, albedo, source, src_sub, npix_x, npix_y,
                          image, stats);
   // the buffers grow to the largest call and stay with the context (about
