@@ -156,15 +156,16 @@ __device__ __forceinline__ double table_at(uint32_t byte) {
 // Predicated adds; written as C++ they become a branch per axis, and the lanes of a
 // warp cross different axes.
 __device__ __forceinline__ void cross_axis(double l, double lmin, double &pos, double moved,
-                                           double face, uint32_t &fi, int fstep, uint32_t &cell,
-                                           int cstep) {
+                                           double &face, uint32_t &fi, int fstep,
+                                           uint32_t &cell, int cstep) {
   asm("{\n\t.reg .pred p;\n\t"
-      "setp.eq.f64 p, %3, %4;\n\t"
-      "selp.f64 %0, %6, %5, p;\n\t"
+      "setp.eq.f64 p, %4, %5;\n\t"
+      "selp.f64 %0, %3, %6, p;\n\t"
       "@p add.s32 %1, %1, %7;\n\t"
+      "@p ld.shared.f64 %3, [%1];\n\t"
       "@p add.s32 %2, %2, %8;\n\t}"
-      : "=d"(pos), "+r"(fi), "+r"(cell)
-      : "d"(l), "d"(lmin), "d"(moved), "d"(face), "r"(fstep), "r"(cstep));
+      : "=d"(pos), "+r"(fi), "+r"(cell), "+d"(face)
+      : "d"(l), "d"(lmin), "d"(moved), "r"(fstep), "r"(cstep));
 }
 __device__ __forceinline__ void cross_axis(float l, float lmin, float &p, float moved,
                                            float &face, float fstep, float fexit, uint32_t &ex,
@@ -521,8 +522,6 @@ struct PathF {
     for (int a = 0; a < 3; ++a)
       cross_axis(l[a], lmin, pos[a], __dadd_rn(pos[a], __dmul_rn(lmin, d[a])), face[a], fi[a],
                  sg[a], cell, cst[a]);
-#pragma unroll
-    for (int a = 0; a < 3; ++a) face[a] = table_at(fi[a]);
     // faces are not negative, so their high words order like integers
     const int top = max(__double2hiint(face[0]),
                         max(__double2hiint(face[1]), __double2hiint(face[2])));
