@@ -1073,8 +1073,6 @@ constexpr int kWgradThreads = kWgradWarps * 32;
 constexpr int kUnitCols = 48;             // one unit's accumulator: taps dx = -1, 0, 1 x 16
 constexpr int kWgradUnitsPerCta = 10;     // 10 x 48 <= 512 TMEM columns
 constexpr int kWgMaxBufs = 4;             // tile buffers in flight at most
-constexpr size_t kWgStaticSmem = 2048;    // static shared memory of a CTA and what the
-                                          // system keeps of it
 
 // dy of a tile with one extra voxel row on either side in y, 16 channels per
 // 32-byte voxel row (32-byte swizzle), x fastest:
@@ -2491,18 +2489,12 @@ int wgrad_t(cmi_unet *u, const Slice &x, const Slice &dy, float *dw, float *db,
     return (std::max(nbuf * buf, reach_end) + 127) / 128 * 128;
   };
   auto smem_for = [&](int nbuf) { return 1024 + bars_at(nbuf) + 128; };
-  // CTAs per SM that the tensor memory allows (the occupancy query answers one for
-  // this kernel) and tile buffers (kWgMaxBufs at most): the most buffers per SM
-  int per_sm = 1;
+  // One CTA per SM.  Two would fit where the units take at most 256 columns (training
+  // step, 64^3 x 8: 2260 -> 2200 us), but each element's FP32 accumulation would then
+  // run over half the tiles: gradients 1.7e-5 from those of one.
   a.nbuf = 1;
-  for (int c = 1; c <= (int)(512 / a.tmem_cols); ++c)
-    for (int nb = 2; nb <= kWgMaxBufs; ++nb)
-      if (smem_for(nb) <= (size_t)optin &&
-          c * (smem_for(nb) + kWgStaticSmem) <= (size_t)optin + kWgStaticSmem &&
-          c * nb >= per_sm * a.nbuf) {
-        per_sm = c;
-        a.nbuf = nb;
-      }
+  for (int nb = 2; nb <= kWgMaxBufs; ++nb)
+    if (smem_for(nb) <= (size_t)optin) a.nbuf = nb;
   a.bar_off = (int)bars_at(a.nbuf);
   const size_t smem = smem_for(a.nbuf);
   if (smem > (size_t)optin)
@@ -2514,7 +2506,7 @@ int wgrad_t(cmi_unet *u, const Slice &x, const Slice &dy, float *dw, float *db,
   UN_CUDA(cudaGetDevice(&dev));
   UN_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   const int tiles = batch * (dims[0] / T::kTX) * (dims[1] / T::kTY) * (dims[2] / T::kTZ);
-  const int ctas = std::max(1, std::min(tiles, per_sm * sms / groups));
+  const int ctas = std::max(1, std::min(tiles, sms / groups));
   // the CTAs' sums go through the network's scratch and one reduction pass when
   // they fit (without it every CTA adds its sums to the same dw entries with
   // FP32 atomics, which costs more than the scratch round trip)
