@@ -69,6 +69,13 @@ constexpr uint32_t kDefaultRefillMixed = 12;
 // 32 copies 2930 / 2620 / 2360, within 6 cells 2860 / 2285 / 2230; one copy 12000.
 constexpr double kHotCells = 5.;
 constexpr uint32_t kTallyCopies = 16;  // a multiple of 8
+// Copies once a source emits kManyPackets.  The lines of one cell's copies share slices
+// of the L2 by chance; more copies even that out, but cost the balance about a
+// microsecond per eight.  16 / 64 copies: log-normal 128^3, 2.5e6 packets per source 2020
+// / 1938 (FP32 2038 / 1904), 64^3, 1e6 from one source 322 / 330, 32^3, 2e4 47 / 55;
+// 128 copies: 1961 (FP32 1825), 256^3 31270 / 32430.
+constexpr uint32_t kTallyCopiesMany = 64;
+constexpr double kManyPackets = 1.5e6;
 constexpr size_t kHotBytes = 64u << 20;
 
 struct HostInstance {
@@ -398,7 +405,7 @@ int plan_tally_copies(cmi_context *c, std::vector<uint32_t> &hot) {
             }
       }
     }
-    copies = kTallyCopies;
+    copies = most >= kManyPackets ? kTallyCopiesMany : kTallyCopies;
     while (copies >= 8 && ((double)(cells * copies * 8) > pays ||
                            c->total_padded + (int64_t)(cells * copies) >= (1ll << 32)))
       copies /= 2;

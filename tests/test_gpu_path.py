@@ -105,3 +105,24 @@ def test_batch_equals_single_instances(precision):
             _, j = eng.get_fields(i, neutral_fraction=False)
             np.testing.assert_allclose(j, 2.0 * jw[i],
                                        rtol=5e-12 if precision == "fp64" else 1e-12, atol=0)
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp32", "fp64"])
+def test_many_packets_of_one_source(precision):
+    """Above 1.5e6 packets of a source its cells have more tally copies.  Up to 1.6e6
+    packets cross a cell: 2 x 1.6e6 x 2^-53 ~ 3.6e-10 for the FP64 sums; the fixed-point
+    ones merge at most 1.6e4 times (1.8e-12, tested at 1e-11)."""
+    for packets in (1_499_999, 1_600_000):
+        g = _grid((16, 16, 16), (2, 2, 2), [(0.4, 0.5, 0.6)], packets, 0.0)
+        nH, xH = _fields(g, 5)
+        with TransportEngine(g, precision=precision) as eng:
+            eng.set_fields(0, nH, xH)
+            ph = eng.emit_photons(seed=91, iteration=2)
+            want = eng.transport_packets(0, ph, _first_subgrids(g, ph))
+            _, jw = eng.get_fields(0, neutral_fraction=False)
+            eng.set_intensity(0, np.zeros(g.num_cells))
+            got = eng.shoot_packets(seed=91, iteration=2)[0]
+            _, jg = eng.get_fields(0, neutral_fraction=False)
+            assert {k: got[k] for k in COUNTS} == {k: want[k] for k in COUNTS}
+            np.testing.assert_allclose(jg, jw, rtol=4e-10 if precision == "fp64" else 1e-11,
+                                       atol=0)
