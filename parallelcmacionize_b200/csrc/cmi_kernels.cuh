@@ -1,9 +1,15 @@
 // Kernels of the B200 transport engine.
 //
-// One iteration of the plain method (testDensitySubGrid_omp.cpp:2213-2434)
-// runs as a wavefront over all instances of a context:
+// One iteration of the plain method (testDensitySubGrid_omp.cpp:2213-2434) over all
+// instances of a context is
 //
-//   emission plan -> emit -> [plan -> scatter -> walk] x R -> balance
+//   begin -> path -> balance
+//
+// where one kernel takes every packet from its source to its end (cmi_path.cuh), or,
+// for given packet lists, ranlxd emission, the FP32 and compensated tally forms and
+// subgrids whose tables do not fit its shared memory, a wavefront:
+//
+//   begin -> emit -> [plan -> scatter -> walk] x R -> balance
 //
 // * emit / walk append packets to an unsorted arena, warp-aggregated: one
 //   atomic per warp for the arena slot and one per group of lanes heading to
@@ -17,8 +23,8 @@
 //   packets one crossing per loop trip, refilling idle lanes; path lengths
 //   are tallied in shared-memory atomics and flushed to the FP64 J array in
 //   HBM once per subgrid residency.
-// R = max over instances of (sum of subgrids per axis - 2), the most subgrid
-// transits a straight ray can make, so no packet is left over.
+// R = max over instances of (sum of subgrids per axis - 2) + 3 spare rounds: the most
+// subgrid transits a straight ray can make, so no packet is left over.
 #pragma once
 
 #include "cmi_device.cuh"

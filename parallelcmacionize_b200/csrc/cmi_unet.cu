@@ -36,11 +36,10 @@
 //    along x x 16 input channels (the B operand's column groups one voxel
 //    apart).  A CTA owns a group of such units, one TMEM accumulator each,
 //    and walks the tiles; per tile it loads dy and the input with its halo by
-//    TMA (the input box of the forward kernel); four warps move dy into TMEM
-//    transposed (lane = output channel), the A operand that every unit's MMAs
-//    share, and the B operand of a unit is the halo at its offset (MN-major).
-//    At the end the accumulators are read with tcgen05.ld and added to dW
-//    with FP32 atomics.
+//    TMA (the input box of the forward kernel); dy shifted by a row in y per
+//    group of 16 rows is the A operand, and the B operand of a unit is the halo
+//    at its offset (both MN-major).  At the end the accumulators are read with
+//    tcgen05.ld and added over the CTAs through scratch.
 //  * pooling, upsampling, activation backward, the 1x1 output head fused
 //    with the MSE loss and its gradient, Adam, weight packing, features.
 #include <cuda.h>
