@@ -531,7 +531,7 @@ def ours(args):
     peak, peak_kind = measured_peak_hbm()
     total_kt = sum(v[0] for v in kt.values())
     roofline = {
-        "kernel": "k_path (emission and walk, %s)" % args.precision,
+        "kernel": ("k_path (emission and walk, %s)" if walk_launches == 1 else "wavefront walk, %s") % args.precision,
         "bound": "hbm", "achieved": achieved,
         "peak": peak, "unit": "GB/s", "frac": achieved / peak, "peak_source": peak_kind,
         "traffic": WALK_TRAFFIC_PER_LAUNCH.get((args.workload, wl.total_packets, args.precision)),

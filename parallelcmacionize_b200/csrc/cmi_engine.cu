@@ -150,7 +150,8 @@ struct cmi_context {
   size_t stage_bytes = 0;
 
   // whole-path transport (cmi_path.cuh) instead of the wavefront, and what it needs
-  bool path = false;
+  bool path_fits = false;  // transport by whole paths is possible ...
+  bool path = false;       // ... and what the present budgets go by (choose_path)
   bool tables_fit = false;  // path_table fits, whatever carries the iterations
   DevGeo *d_geo = nullptr;
   unsigned long long *d_tally = nullptr;
@@ -446,6 +447,24 @@ bool ensure_pair(cmi_context *c) {
   return c->d_pair != nullptr;
 }
 
+// Whole paths, but for the FP32 walk through so many cells that opacities and tallies
+// (12 bytes per cell) are far larger than the L2, with packets enough to fill the chunks of
+// large subgrids.  There every reduction of k_path misses, while the wavefront tallies in
+// shared memory.  B200, ms per iteration, paths / wavefront: 64 instances, 4.7e7 cells,
+// 2.4e8 packets 70.0 / 58.6; 256^3 in 16^3 subgrids, 16 sources, 1e8 packets 39.9 / 39.2
+// (sigma_ln 1.5: 55.4 / 52.5), 4e7 packets 16.3 / 16.4, in 8^3 subgrids, 1e8 packets
+// 45.9 / 55.0; 224^3, 4e7 packets 14.1 / 15.4.  With reemission the path kernel's lead is
+// far larger (64^3, mixed: 0.64 / 3.1).
+constexpr int64_t kWavefrontCells = 14000000;
+constexpr int64_t kWavefrontSubgrid = 2048;  // cells per subgrid on average
+constexpr uint64_t kWavefrontPackets = 4;    // per cell
+bool choose_path(const cmi_context *c) {
+  const bool wavefront = c->fp32() && !c->reemission && c->total_padded >= kWavefrontCells &&
+                         c->total_padded / c->S >= kWavefrontSubgrid &&
+                         total_budget(c) >= kWavefrontPackets * (uint64_t)c->total_padded;
+  return c->path_fits && !wavefront;
+}
+
 // Upload instance + source tables (after sources or budgets change).
 int upload_tables(cmi_context *c) {
   bool reemission = false;
@@ -518,6 +537,7 @@ int upload_tables(cmi_context *c) {
                            cudaMemcpyHostToDevice, c->stream));
   std::vector<DevGeo> geo;
   std::vector<uint32_t> hot;
+  c->path = choose_path(c);
   if (c->path) {
     CMI_TRY(plan_tally_copies(c, hot));
     CMI_CUDA(cudaMemcpyAsync(c->d_hot, hot.data(), sizeof(uint32_t) * hot.size(),
@@ -768,7 +788,7 @@ int config_path_kernels(cmi_context *c) {
 // FP64, 64^3 at 4 / 5 / 6 249 / 243 / 265; FP32, 96 x 80 x 112 at 7 / 8 / 9 707 / 718 / 779)
 constexpr int kPathMinM = 6, kPathMin32 = 8, kPathMin64 = 5;
 int config_path(cmi_context *c) {
-  if (!c->path) return CMI_OK;
+  if (!c->path_fits) return CMI_OK;
   if (c->fp32()) return config_path_kernels<Path32<true>, Path32<false>, kPathMin32>(c);
   if (c->mixed()) return config_path_kernels<PathF<true, true>, PathF<true, false>, kPathMinM>(c);
   return config_path_kernels<PathF<false, true>, PathF<false, false>, kPathMin64>(c);
@@ -1261,7 +1281,7 @@ int cmi_create(const cmi_grid_desc *grids, int32_t num_instances, const cmi_opti
     c->path_table = std::max(c->path_table, instance_geometry(c, I).table);
   c->path_smem = (sizeof(PathShared) + sizeof(double) * (size_t)c->path_table) * kPathWarps;
   c->tables_fit = c->total_padded < (1ll << 31) && c->path_smem <= kPathSmemMost;
-  c->path = c->tables_fit && opt.rng == CMI_RNG_PHILOX &&
+  c->path_fits = c->tables_fit && opt.rng == CMI_RNG_PHILOX &&
             (c->fp64() || opt.tally_mode == CMI_TALLY_FIXED64 ||
              opt.tally_mode == CMI_TALLY_FIXED64_ATOMIC64);
 
