@@ -25,11 +25,11 @@
 // * Lanes at a face, done and free ones wait until several do (kTransit and kRefill of
 //   the lane state); packets are emitted 32 at a time into a queue.
 //
-// Bound by instruction issue and lane divergence (log-normal 128^3, mixed: 54% of
-// issue slots, 19 of 32 lanes, L1 58% and L2 37% of peak).  Against the wavefront, us
-// per iteration: 32^3, 2e4 packets 216 -> 60; stromgren 64^3, 1e6 907 -> 335;
-// log-normal 128^3, 1e7 4060 -> 2034; 256^3, 1e8 53000 -> 32400; 12 uneven instances
-// 6860 -> 4050; FP64 walk, 64^3, 1e6 1276 -> 242.
+// Bound by instruction issue and lane divergence (log-normal 128^3, mixed, 4e6 packets:
+// 63% of issue slots, 19 of 32 lanes, L1 73% of peak, L2 48% and 95% in its busiest
+// slice).  Against the wavefront, us per iteration: 32^3, 2e4 packets 214 -> 57;
+// stromgren 64^3, 1e6 913 -> 329; log-normal 128^3, 1e7 3800 -> 2005; 256^3, 1e8
+// 79100 -> 54300; 12 uneven instances 7170 -> 4200; FP64 walk, 64^3, 1e6 1561 -> 280.
 #pragma once
 
 #include "cmi_kernels.cuh"
